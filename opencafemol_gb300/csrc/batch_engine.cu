@@ -8,14 +8,16 @@
 // list entries beyond the shared-memory share and L2-resident parameters.
 // Per MD step:
 //   list:     Verlet lists with a 0.3 nm skin, rebuilt when a bead has
-//             moved more than half the skin (one thread per bead, j order);
-//   forces:   pair units (a bead and a j-range of its list) write the
-//             bead's pair force; one lane per chain position evaluates the
+//             moved more than half the skin: one list per pair unit (a bead
+//             and a j-range, one thread each, j order), and one per charged
+//             bead of its charged partners;
+//   forces:   pair units write the bead's pair force, charged units its
+//             Debye-Hueckel force; one lane per chain position evaluates the
 //             chain-local bonded terms starting there and the lanes combine
 //             them by shuffles; other bonded terms are gathered by each of
 //             their beads;
-//   update:   Langevin step per bead from the summed forces, bounding boxes,
-//             displacement and blow-up checks.
+//   update:   Langevin step per bead from the summed forces, displacement
+//             and blow-up checks.
 // No atomics on forces: every bead's force is a sum in a fixed order, so a
 // system gives the same trajectory alone, in any mix, for any chunking and
 // for any threads per CTA.
@@ -42,31 +44,62 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxClusters = 64;  // 2048 beads per system
 // Pair work of a bead is split over S adjacent lanes (S = 1, 2, 4 or 8, the
-// largest with n * S <= kSplitUnits); sub-lane s sums the list entries whose
-// j lies in [s*n/S, (s+1)*n/S).  S depends on n alone, so the FP32 sums, and
+// largest with n * S <= kSplitUnits); sub-lane s sums the partners whose j
+// lies in [s*n/S, (s+1)*n/S).  S depends on n alone, so the FP32 sums, and
 // the results, do not depend on the threads per CTA (a CTA with fewer
-// threads walks the units in more passes).
+// threads walks the units in more passes).  The charged beads' partners are
+// split the same way among the nq charged beads (kSplitCharged).
 constexpr int kSplitUnits = 512;
-constexpr int kMaxUnits = kSplitUnits;
+constexpr int kSplitCharged = 128;
 constexpr int kMaxSplit = 8;
-// Beads are ordered by their longest sub-list at every list build (bucket
-// sort over this many buckets), so the 32 lanes of a pair pass carry work of
-// similar length.
+// Beads are ordered by their longest sub-list (bucket sort over this many
+// buckets), so the 32 lanes of a pair pass carry work of similar length.
+// The order is taken from the last lists of a launch and of every
+// kSortBuilds-th build within it, and is kept between launches.
 constexpr int kSortBuckets = 64;
+constexpr int kSortBuilds = 4;
+
+// Classes of systems by their pair terms; each has its own list layout and
+// inner loop, chosen per system, so a system's results do not depend on
+// which other classes a launch holds.
+//   Go:      excluded volume and Debye-Hueckel, no interaction groups.
+//   Hps:     both Lennard-Jones terms (one sigma per bead, arithmetic
+//            epsilon, one cutoff, the same excluded pairs) and
+//            Debye-Hueckel, no interaction groups.
+//   General: everything else.
+// Go and Hps keep two plain lists, the partners that interact by the
+// short-range term and, per charged bead, the charged partners within the
+// Debye-Hueckel cutoff: no exclusion bits, no charge test per pair, and a
+// long Debye-Hueckel cutoff lengthens the charged beads' lists alone (300
+// disordered chains of 50..400 beads, 3.5 nm against 2.0 nm: one combined
+// list holds about 2.5 times as many entries).  General keeps one list whose
+// entries carry the excluded terms.
+// Issue-bound: an excluded-volume entry takes about 23 instructions and one
+// 16-byte gather where the combined walk took over 40 and two.  Per 100 steps
+// with the read-out, against one combined list for all: 512 Go proteins of
+// 50..800 beads 2.92 -> 2.30 ms, 300 disordered chains 6.74 -> 1.95 ms, 24
+// proteins of 30..200 beads 0.84 -> 0.56 ms; per 50 steps 160 AICG2+
+// proteins of 800..2000 beads 3.94 -> 2.86 ms (these also through bonds kept
+// chain-local to three positions).
+constexpr int kClassGo = 0;
+constexpr int kClassHps = 1;
+constexpr int kClassGeneral = 2;
+
 // Shared memory of a system: bytes per bead (state, lists' counts, order)
-// and the part that does not grow with the bead count (cluster boxes and
-// carries, pair-split offsets, sort buckets, alignment).
-constexpr int kBeadBytes = 100;
-constexpr int kBeadBytesGeneral = 120;  // with per-bead LJ attraction parameters and labels
-constexpr size_t kFixedBytes = (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kMaxUnits + 4 * kSortBuckets;
+// and the part that does not grow with the bead count (the dummy bead, the
+// cluster boxes and carries, the unit counts of small systems, the sort
+// buckets, alignment).
+constexpr int kBeadBytes[3] = {104, 112, 120};
+constexpr size_t kFixedBytes =
+    (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kSplitUnits + 2 * kSplitCharged + 4 * kSortBuckets + 16;
 // A force component beyond this (kJ/mol/nm) marks a blown-up system: far
 // above any physical coarse-grained force, and the bound of the plain
 // engine's fixed-point accumulators.
 constexpr float kForceLimit = 1.0e9f;
 
-__host__ __device__ __forceinline__ int pair_split(int n) {
+__host__ __device__ __forceinline__ int pair_split(int n, int units) {
     int S = 1;
-    while (S < kMaxSplit && n * S * 2 <= kSplitUnits) S <<= 1;
+    while (S < kMaxSplit && n * S * 2 <= units) S <<= 1;
     return S;
 }
 
@@ -84,6 +117,7 @@ struct BatchArgs {
     double* energy;              // [slot][kNumSlots]
     float* forces;               // eval output [3][nmax]
     uint16_t* lists;             // neighbour-list arena
+    uint16_t* bead_order;        // per bead arena: the systems' bead order of the pair passes
     uint32_t slots_enabled;
     size_t smem_bytes;           // dynamic shared memory of the launch
     int split_beads;             // a CTA splits into two groups at systems of at most this many beads (0: never)
@@ -213,8 +247,8 @@ __device__ __forceinline__ void dihedral_force(const Bonded& B, int q, const flo
 __device__ __forceinline__ bool slot_on(uint32_t slots_en, int slot) { return (slots_en >> slot) & 1u; }
 
 // Bonded force on bead b = I * 32 + lane of cluster I (one warp).  The lane
-// evaluates every chain-local term starting at b (bonds b-b+1, angles
-// b..b+2, dihedrals b..b+3) once, keeping its contributions to b..b+3; the
+// evaluates every chain-local term starting at b (bonds from b to b+1, b+2
+// or b+3, angles b..b+2, dihedrals b..b+3) once, keeping its contributions to b..b+3; the
 // lanes then add what lanes 1..3 below them send up, in a fixed order, and
 // the three contributions that cross into cluster I + 1 go to carry[I].
 // Terms that are not chain-local are evaluated by each of their beads
@@ -232,7 +266,10 @@ __device__ __forceinline__ float3 bonded_cluster(const Bonded& B, int I, int n, 
             const float3 f = bond_force(B, t, sx, sxl, ns, en, sl);
             if (!slot_on(slots_en, sl)) continue;
             add3(o0, f);
-            add3(o1, neg3(f));
+            const int d = (int)((B.bij[t] >> 16) & 0x3FFF) - b;
+            if (d == 1) add3(o1, neg3(f));
+            else if (d == 2) add3(o2, neg3(f));
+            else add3(o3, neg3(f));
             if (ENERGY) ea.e[sl] += (double)en;
         }
         if (slot_on(slots_en, kSlotFLA))
@@ -356,82 +393,171 @@ __device__ __forceinline__ uint32_t label_bits(uint32_t labi, uint32_t labj, con
     return bits;
 }
 
-// Neighbour list of every bead of the claimed system, built by one thread
-// per bead: all j != i whose FP32 r^2 (canonical form) is below cut2, in
-// increasing j, so the list and every FP32 sum over it are deterministic.
-// Entry = j | (excluded-term bits << 11); pairs excluded for every present
-// term are dropped.  Entry k of bead i lives in shared memory at
-// slist[k * npad + i] for k < cap_s and in global memory at
-// glist[k * npad + i] for cap_s <= k < maxn.  Sets *overflow when a list
-// exceeds maxn.  Then bord = the beads in decreasing length of their
-// longest sub-list (bucket sort; ties in any order), through the group's
-// barrier `bar`; tmp (n words) and hist (kSortBuckets words, zero on entry
-// and on return) are scratch.
-template <bool LABELS>
-__device__ __forceinline__ void build_lists(int n, int nt, int npad, int maxn, int cap_s, float cut2,
-                                            const float4* sx, const uint32_t* slab,
-                                            const float4* bc, const float4* bh,
-                                            const int32_t* __restrict__ ex_start,
-                                            const int32_t* __restrict__ ex,
-                                            const PairConsts& pc, uint16_t* slist,
-                                            uint16_t* __restrict__ glist, uint16_t* scnt,
-                                            float* sref, int nmax, int tid, int threads,
-                                            int S, uint16_t* sseg, int* overflow, uint16_t* bord,
-                                            int* hist, uint32_t* tmp, int bar) {
-    const float3 nobox = make_float3(0.f, 0.f, 0.f);
+// Columns of a list over m beads, each split into S units: whole warps.
+__host__ __device__ __forceinline__ int list_columns(int m, int S) { return (m * S + 31) & ~31; }
+
+// Lists of one kind: a column of at most `cap` entries per unit, entry k of
+// column c at ((k / 4) * cols + c) * 4 + k % 4, so a lane reads four entries
+// with one 8-byte load and the lanes of a pass read consecutive words.  The
+// first cap_s entries of a column live in shared memory, the rest in global
+// memory; both capacities are multiples of 4, and a column is filled up to
+// whole groups of four with entries that contribute nothing.
+struct UnitList {
+    uint16_t *s, *g;
+    int cap_s, cap, cols;
+};
+
+__device__ __forceinline__ void list_put(const UnitList& L, int k, int col, uint32_t e) {
+    const size_t at = ((size_t)(k >> 2) * L.cols + col) * 4 + (k & 3);
+    if (k < L.cap_s) L.s[at] = (uint16_t)e;
+    else if (k < L.cap) L.g[at] = (uint16_t)e;
+}
+
+// Pads the last group and returns the stored count.
+__device__ __forceinline__ int list_close(const UnitList& L, int k, int col, uint32_t pad, int* overflow) {
+    if (k > L.cap) {
+        atomicOr(overflow, 1);
+        return L.cap;
+    }
+    for (int q = k; q & 3; ++q) list_put(L, q, col, pad);
+    return k;
+}
+
+// Groups of four entries of a column, in order.
+template <class F>
+__device__ __forceinline__ void list_walk(const UnitList& L, int col, int cnt, F&& four) {
+    const int groups = (cnt + 3) >> 2, shared = min(groups, L.cap_s >> 2);
+    const uint16_t* p = L.s + (size_t)col * 4;
+    for (int g = 0; g < shared; ++g) four(*reinterpret_cast<const uint2*>(p + (size_t)g * L.cols * 4));
+    const uint16_t* q = L.g + (size_t)col * 4;
+    for (int g = shared; g < groups; ++g) four(*reinterpret_cast<const uint2*>(q + (size_t)g * L.cols * 4));
+}
+
+__device__ __forceinline__ uint32_t entry_of(uint2 e, int u) {
+    const uint32_t w = u < 2 ? e.x : e.y;
+    return u & 1 ? w >> 16 : w & 0xFFFFu;
+}
+
+// Whether bead x is at least sqrt(cut2) away from cluster J's bounding box.
+__device__ __forceinline__ bool box_far(float4 x, float4 c, float4 h, float cut2) {
+    const float gx = fmaxf(0.f, fabsf(x.x - c.x) - h.x);
+    const float gy = fmaxf(0.f, fabsf(x.y - c.y) - h.y);
+    const float gz = fmaxf(0.f, fabsf(x.z - c.z) - h.z);
+    return gx * gx + gy * gy + gz * gz >= cut2;
+}
+
+// Main list of every unit, one thread per unit (bead i, range s): the j != i
+// of the range whose FP32 r^2 (canonical form) is below cut2, in increasing
+// j, so the list and every FP32 sum over it are deterministic.  Go and Hps
+// keep j alone and leave out the pairs that their short-range term excludes;
+// General keeps j | excluded-term bits << 11 and leaves out the pairs that
+// every present term excludes.  Per cluster the 32 distance tests set bits
+// of a mask without a branch and only the set bits go on, with the
+// exclusions taken out first: with a test and an exclusion walk per j the
+// warp took the hit path for almost every j.
+// The unit's column is that of its bead in the pass order (pos[i]), so the
+// lanes of a pass find their entries side by side.
+template <int CLS>
+__device__ __forceinline__ void build_main(int n, int lg, float cut2, const float4* sx, const uint32_t* slab,
+                                           const float4* bc, const float4* bh,
+                                           const int32_t* __restrict__ ex_start, const int32_t* __restrict__ ex,
+                                           const PairConsts& pc, const UnitList& L, const uint16_t* pos,
+                                           uint16_t* ucnt, int npad, int tid, int threads, int* overflow) {
     const uint32_t present = (uint32_t)pc.terms;
-    for (int i = tid; i < n; i += threads) {
+    const int32_t drop = (CLS == kClassGo ? kTermEXV : kTermLJR) << 24;
+    for (int u = tid; u < n << lg; u += threads) {
+        const int i = u >> lg, s = u & ((1 << lg) - 1);
+        const int j0 = (s * n) >> lg, j1 = ((s + 1) * n) >> lg;
+        const int col = ((int)pos[i] << lg) + s;
         const float4 xi = sx[i];
-        const uint32_t labi = LABELS ? slab[i] : 0u;
-        int cnt = 0;
-        int seg0 = 0, longest = 0;  // start of the current sub-list, longest so far
-        // list offset where each j-range of the pair split starts
-        int s_next = 1;
-        int jb = S > 1 ? n / S : 0x7FFFFFFF;
-        if (S > 1) sseg[i * S] = 0;
+        const uint32_t labi = CLS == kClassGeneral ? slab[i] : 0u;
         int ep = ex_start[i];
         const int e1 = ex_start[i + 1];
-        int ej = ep < e1 ? (ex[ep] & 0xFFFFFF) : 0x7FFFFFFF;
-        for (int J = 0; J < nt; ++J) {
-            const float4 c = bc[J], h = bh[J];
-            const float gx = fmaxf(0.f, fabsf(xi.x - c.x) - h.x);
-            const float gy = fmaxf(0.f, fabsf(xi.y - c.y) - h.y);
-            const float gz = fmaxf(0.f, fabsf(xi.z - c.z) - h.z);
-            if (gx * gx + gy * gy + gz * gz >= cut2) continue;
-            const int j1 = min(n, J * 32 + 32);
-            for (int j = J * 32; j < j1; ++j) {
-                if (j == i) continue;
-                const float r2 = norm2(separation<false>(xi, sx[j], nobox, nobox));
-                if (!(r2 < cut2)) continue;
-                uint32_t bits = excl_walk(j, ep, ej, e1, ex);
-                if (LABELS) bits |= label_bits<true>(labi, slab[j], pc);
-                if ((bits & present) == present) continue;
-                while (j >= jb) {
-                    const int c = min(cnt, maxn);
-                    longest = max(longest, c - seg0);
-                    seg0 = c;
-                    sseg[i * S + s_next] = (uint16_t)c;
-                    ++s_next;
-                    jb = s_next < S ? (s_next * n) / S : 0x7FFFFFFF;
+        int32_t ew = ep < e1 ? ex[ep] : 0x00FFFFFF;  // the next exclusion at or after the walk
+        int cnt = 0;
+        for (int jb = j0 & ~31; jb < j1; jb += 32) {
+            if (box_far(xi, bc[jb >> 5], bh[jb >> 5], cut2)) continue;
+            uint32_t m = 0u;
+#pragma unroll 8
+            for (int t = 0; t < 32; ++t) {
+                const float4 xj = sx[jb + t];
+                const float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y), dz = __fsub_rn(xj.z, xi.z);
+                m |= (norm2(make_float3(dx, dy, dz)) < cut2 ? 1u : 0u) << t;
+            }
+            if (jb < j0) m &= 0xFFFFFFFFu << (j0 - jb);
+            if (j1 - jb < 32) m &= (1u << (j1 - jb)) - 1u;
+            if (i >> 5 == jb >> 5) m &= ~(1u << (i & 31));
+            while ((ew & 0xFFFFFF) < jb) ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
+            if (CLS != kClassGeneral) {
+                while ((ew & 0xFFFFFF) < jb + 32) {
+                    if (ew & drop) m &= ~(1u << ((ew & 0xFFFFFF) - jb));
+                    ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
                 }
-                const uint16_t e = (uint16_t)(j | (bits << 11));
-                if (cnt < cap_s) slist[cnt * npad + i] = e;
-                else if (cnt < maxn) glist[(size_t)cnt * npad + i] = e;
-                ++cnt;
+                for (; m; m &= m - 1) list_put(L, cnt++, col, (uint32_t)(jb + __ffs(m) - 1));
+            } else {
+                for (; m; m &= m - 1) {
+                    const int j = jb + __ffs(m) - 1;
+                    while ((ew & 0xFFFFFF) < j) ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
+                    uint32_t bits = (ew & 0xFFFFFF) == j ? (uint32_t)ew >> 24 : 0u;
+                    bits |= label_bits<true>(labi, slab[j], pc);
+                    if ((bits & present) != present) list_put(L, cnt++, col, (uint32_t)j | bits << 11);
+                }
             }
         }
-        if (cnt > maxn) {
-            atomicOr(overflow, 1);
-            cnt = maxn;
+        // padding: the dummy bead, or the bead itself with every term excluded
+        ucnt[col] = (uint16_t)list_close(L, cnt, col, CLS == kClassGeneral ? (uint32_t)i | 15u << 11 : (uint32_t)npad,
+                                         overflow);
+    }
+}
+
+// Charged list of every charged unit (charged bead c, range s of the charged
+// beads): the charged j != i within the Debye-Hueckel list cutoff that its
+// exclusions keep, in increasing j.
+__device__ __forceinline__ void build_charged(int nq, int lg, float cut2, const float4* sx, const uint16_t* qidx,
+                                              const int32_t* __restrict__ ex_start,
+                                              const int32_t* __restrict__ ex, const UnitList& L, uint16_t* qcnt,
+                                              int npad, int tid, int threads, int* overflow) {
+    for (int u = tid; u < nq << lg; u += threads) {
+        const int c = u >> lg, s = u & ((1 << lg) - 1);
+        const int c0 = (s * nq) >> lg, c1 = ((s + 1) * nq) >> lg;
+        const int i = qidx[c];
+        const float4 xi = sx[i];
+        int ep = ex_start[i];
+        const int e1 = ex_start[i + 1];
+        int32_t ew = ep < e1 ? ex[ep] : 0x00FFFFFF;
+        int cnt = 0;
+        for (int cb = c0; cb < c1; cb += 32) {
+            uint32_t m = 0u;
+            const int end = min(32, c1 - cb);
+#pragma unroll 4
+            for (int t = 0; t < end; ++t) {
+                const float4 xj = sx[qidx[cb + t]];
+                const float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y), dz = __fsub_rn(xj.z, xi.z);
+                m |= (norm2(make_float3(dx, dy, dz)) < cut2 ? 1u : 0u) << t;
+            }
+            for (; m; m &= m - 1) {
+                const int j = qidx[cb + __ffs(m) - 1];
+                if (j == i) continue;
+                while ((ew & 0xFFFFFF) < j) ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
+                if ((ew & 0xFFFFFF) == j && (ew & kTermDH << 24)) continue;
+                list_put(L, cnt++, u, (uint32_t)j);
+            }
         }
-        for (; s_next < S; ++s_next) sseg[i * S + s_next] = (uint16_t)cnt;
-        scnt[i] = (uint16_t)cnt;
-        sref[i] = xi.x;
-        sref[nmax + i] = xi.y;
-        sref[2 * nmax + i] = xi.z;
-        longest = max(longest, cnt - seg0);
+        qcnt[u] = (uint16_t)list_close(L, cnt, u, (uint32_t)npad, overflow);
+    }
+}
+
+// New bead order of the pair passes: decreasing length of a bead's longest
+// sub-list (bucket sort; ties in any order).  tmp (n words), out (n
+// half-words) and hist (kSortBuckets words, zero on entry and on return) are
+// scratch; ends with a barrier.
+__device__ __forceinline__ void sort_beads(int n, int lg, const uint16_t* ucnt, uint16_t* bord, int* hist,
+                                           uint32_t* tmp, uint16_t* out, int tid, int threads, int bar) {
+    for (int p = tid; p < n; p += threads) {
+        int longest = 0;
+        for (int s = 0; s < 1 << lg; ++s) longest = max(longest, (int)ucnt[(p << lg) + s]);
         const int bucket = longest < 32 ? longest : min(kSortBuckets - 1, 32 + ((longest - 32) >> 2));
-        tmp[i] = (uint32_t)bucket | (uint32_t)atomicAdd(&hist[bucket], 1) << 8;
+        tmp[p] = (uint32_t)bucket | (uint32_t)atomicAdd(&hist[bucket], 1) << 8;
     }
     bar_sync(bar, threads);
     if (tid < 32) {
@@ -449,149 +575,273 @@ __device__ __forceinline__ void build_lists(int n, int nt, int npad, int maxn, i
         hist[kSortBuckets - 2 - 2 * tid] = incl - pair + h0;
     }
     bar_sync(bar, threads);
-    for (int i = tid; i < n; i += threads) {
-        const uint32_t t = tmp[i];
-        bord[hist[t & 255u] + (int)(t >> 8)] = (uint16_t)i;
+    for (int p = tid; p < n; p += threads) {
+        const uint32_t t = tmp[p];
+        out[hist[t & 255u] + (int)(t >> 8)] = bord[p];
     }
     bar_sync(bar, threads);
-    if (tid < kSortBuckets) hist[tid] = 0;
+    for (int p = tid; p < n; p += threads) bord[p] = out[p];
+    for (int k = tid; k < kSortBuckets; k += threads) hist[k] = 0;
+    bar_sync(bar, threads);
 }
 
-template <int TERMS, bool ENERGY>
-__device__ __forceinline__ void pair_accumulate(int i, int j, float4 xi, float4 xj, float4 p0i, float4 p1i,
-                                                const float4* sp0, const float4* sp1, uint32_t bits,
-                                                const PairConsts& pc, float3& fa, EnergyAcc& ea) {
+// ---------------------------------------------------------------------------
+// Pair arithmetic of the Go and Hps classes.  Every operation is rounded by
+// itself, so the list walk, the scan and every kernel that holds a class
+// give the same bits.  A pair outside the cutoff contributes exactly zero.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ void sub_force(float3& f, float s, float3 d) {
+    f.x = __fmaf_rn(-s, d.x, f.x);
+    f.y = __fmaf_rn(-s, d.y, f.y);
+    f.z = __fmaf_rn(-s, d.z, f.z);
+}
+
+// Excluded volume; .w of a position is the bead's radius.
+template <bool ENERGY>
+__device__ __forceinline__ void exv_pair(float4 xi, float4 xj, const PairConsts& pc, float3& f, EnergyAcc& ea) {
+    const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
+    const float r2 = norm2(d);
+    const bool in = r2 < pc.exv_rc2;
+    const float ri = rcp_approx(in ? r2 : 1.f);
+    const float S = __fadd_rn(xi.w, xj.w);
+    const float S2 = __fmul_rn(S, S);
+    const float u = __fmul_rn(S2, ri);
+    const float u3 = __fmul_rn(__fmul_rn(u, u), u);
+    const float u6 = __fmul_rn(u3, u3);
+    const float s = __fmul_rn(__fmul_rn(__fmul_rn(12.f, pc.exv_eps), u6), ri);
+    sub_force(f, in ? s : 0.f, d);
+    if (ENERGY && in) {
+        const float w = S2 * pc.exv_inv_rc2;
+        const float w3 = w * w * w;
+        ea.e[kSlotEXV] += 0.5 * (double)(pc.exv_eps * (u6 - w3 * w3));  // a pair is met from both of its beads
+    }
+}
+
+// Both Lennard-Jones terms; .w of a position is half the bead's sigma, le
+// half its repulsive and attractive epsilon.  Inside the core (r <= 2^(1/6)
+// sigma) the repulsive term acts and the attractive one is flat, outside the
+// attractive one alone, so one power form serves both.
+template <bool ENERGY>
+__device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float2 lej, const PairConsts& pc, float3& f,
+                                         EnergyAcc& ea) {
+    const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
+    const float r2 = norm2(d);
+    const bool in = r2 < pc.lja_rc2;
+    const float r2c = in ? r2 : 1.f;
+    const float rinv = rsqrtf(r2c);
+    const float ri = __fmul_rn(rinv, rinv);
+    const float sg = __fadd_rn(xi.w, xj.w);
+    const float sig2 = __fmul_rn(sg, sg);
+    const float s2 = __fmul_rn(sig2, ri);
+    const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+    const float s12 = __fmul_rn(s6, s6);
+    const bool core = r2c <= __fmul_rn(sig2, kTwoPow1_3);
+    const float er = __fadd_rn(lei.x, lej.x), el = __fadd_rn(lei.y, lej.y);
+    const float t = __fmul_rn(__fmul_rn(24.f, ri), __fmaf_rn(2.f, s12, -s6));
+    float s = __fmul_rn(core ? er : el, t);
+    const float r = __fmul_rn(r2c, rinv);
+    float sw = 1.f;
+    if (r > pc.lja_rs) {
+        // OpenMM switching function S = 1 - 10x^3 + 15x^4 - 6x^5.
+        const float x = __fmul_rn(__fsub_rn(r, pc.lja_rs), pc.lja_inv_width);
+        const float x2 = __fmul_rn(x, x);
+        const float x3 = __fmul_rn(x2, x);
+        sw = __fmaf_rn(x3, __fmaf_rn(x, __fmaf_rn(-6.f, x, 15.f), -10.f), 1.f);
+        const float dsw = __fmul_rn(__fmul_rn(x2, __fmaf_rn(x, __fmaf_rn(-30.f, x, 60.f), -30.f)), pc.lja_inv_width);
+        const float E = core ? -el : __fmul_rn(__fmul_rn(4.f, el), __fsub_rn(s12, s6));
+        const float att = __fmaf_rn(core ? 0.f : s, sw, -__fmul_rn(__fmul_rn(E, dsw), rinv));
+        s = __fadd_rn(core ? s : 0.f, att);
+    }
+    sub_force(f, in ? s : 0.f, d);
+    if (ENERGY && in) {
+        const float e4 = 4.f * (s12 - s6);
+        if (core) ea.e[kSlotLJR] += 0.5 * (double)(er * (e4 + 1.f));
+        ea.e[kSlotLJA] += 0.5 * (double)((core ? -el : el * e4) * sw);
+    }
+}
+
+// Debye-Hueckel between charges, qk = q_i k_e.
+template <bool ENERGY>
+__device__ __forceinline__ void dh_pair(float4 xi, float4 xj, float qk, float qj, const PairConsts& pc, float3& f,
+                                        EnergyAcc& ea) {
+    const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
+    const float r2 = norm2(d);
+    const bool in = r2 < pc.dh_rc2;
+    const float r2c = in ? r2 : 1.f;
+    const float rinv = rsqrtf(r2c);
+    const float ri = __fmul_rn(rinv, rinv);
+    const float ex = exp2f(__fmul_rn(-__fmul_rn(r2c, rinv), pc.dh_inv_lambda_log2e));
+    const float qq = __fmul_rn(qk, qj);
+    const float s = __fmul_rn(__fmul_rn(__fmul_rn(qq, ex), __fadd_rn(pc.dh_inv_lambda, rinv)), ri);
+    sub_force(f, in ? s : 0.f, d);
+    if (ENERGY && in) ea.e[kSlotDH] += 0.5 * (double)(qq * (ex * rinv - pc.dh_corr));
+}
+
+template <bool ENERGY>
+__device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 p0i, float4 p0j, float4 p1i, float4 p1j,
+                                             uint32_t bits, const PairConsts& pc, float3& fa, EnergyAcc& ea) {
     const float3 nobox = make_float3(0.f, 0.f, 0.f);
     const float3 d = separation<false>(xi, xj, nobox, nobox);
     const float r2 = norm2(d);
-    if (r2 < pc.list_rc2) {
-        const float4 p0j = sp0[j];
-        const float4 p1j = (TERMS & kTermLJA) ? sp1[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        PairEnergy e;
-        e.zero();
-        const float s = pair_scalar<TERMS, ENERGY>(r2, p0i, p0j, p1i, p1j, bits, pc, e);
-        fa.x -= s * d.x;
-        fa.y -= s * d.y;
-        fa.z -= s * d.z;
-        if (ENERGY) {
-            // every pair is met from both of its beads
-            ea.e[kSlotEXV] += 0.5 * (double)e.exv;
-            ea.e[kSlotDH] += 0.5 * (double)e.dh;
-            ea.e[kSlotLJR] += 0.5 * (double)e.ljr;
-            ea.e[kSlotLJA] += 0.5 * (double)e.lja;
-        }
+    const bool in = r2 < pc.list_rc2;
+    PairEnergy e;
+    e.zero();
+    float sc = pair_scalar<15, ENERGY>(in ? r2 : pc.list_rc2, p0i, p0j, p1i, p1j, bits, pc, e);
+    sc = in ? sc : 0.f;
+    fa.x -= sc * d.x;
+    fa.y -= sc * d.y;
+    fa.z -= sc * d.z;
+    if (ENERGY && in) {
+        // every pair is met from both of its beads
+        ea.e[kSlotEXV] += 0.5 * (double)e.exv;
+        ea.e[kSlotDH] += 0.5 * (double)e.dh;
+        ea.e[kSlotLJR] += 0.5 * (double)e.ljr;
+        ea.e[kSlotLJA] += 0.5 * (double)e.lja;
     }
 }
 
-// Pair forces of list entries [k0, k1) of bead i in one memory space,
-// four entries per iteration: the entries' loads are issued first, and the
-// cutoff test selects the result instead of branching, so the four pair
-// evaluations interleave.  One accumulator in list (= increasing j) order:
-// entries outside the cutoff contribute exactly zero.
-template <int TERMS, bool ENERGY>
-__device__ __forceinline__ void list_range(int i, int k0, int k1, int npad, const uint16_t* __restrict__ L,
-                                           float4 xi, float4 p0i, float4 p1i, const float4* sx,
-                                           const float4* sp0, const float4* sp1, uint32_t excl_all,
-                                           const PairConsts& pc, float3& fa, EnergyAcc& ea) {
-    const float3 nobox = make_float3(0.f, 0.f, 0.f);
-    for (int k = k0; k < k1; k += 4) {
-        uint32_t ent[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) ent[u] = k + u < k1 ? (uint32_t)L[(size_t)(k + u) * npad + i] : (uint32_t)i;
-        float4 xj[4], p0j[4], p1j[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = (int)(ent[u] & 2047u);
-            xj[u] = sx[j];
-            p0j[u] = sp0[j];
-            p1j[u] = (TERMS & kTermLJA) ? sp1[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float3 d = separation<false>(xi, xj[u], nobox, nobox);
-            const float r2 = norm2(d);
-            const bool in = k + u < k1 && r2 < pc.list_rc2;
-            PairEnergy e;
-            e.zero();
-            float sc = pair_scalar<TERMS, ENERGY>(in ? r2 : pc.list_rc2, p0i, p0j[u], p1i, p1j[u],
-                                                  (ent[u] >> 11) | excl_all, pc, e);
-            sc = in ? sc : 0.f;
-            fa.x -= sc * d.x;
-            fa.y -= sc * d.y;
-            fa.z -= sc * d.z;
-            if (ENERGY && in) {
-                // every pair is met from both of its beads
-                ea.e[kSlotEXV] += 0.5 * (double)e.exv;
-                ea.e[kSlotDH] += 0.5 * (double)e.dh;
-                ea.e[kSlotLJR] += 0.5 * (double)e.ljr;
-                ea.e[kSlotLJA] += 0.5 * (double)e.lja;
-            }
-        }
-    }
-}
+// Per-bead parameters of the pair terms as staged in shared memory.
+struct PairParams {
+    const float4 *p0, *p1;  // General
+    const uint32_t* lab;    // General
+    const float2* le;       // Hps
+    const float* q;         // Go and Hps: charges
+};
 
-// Pair forces on bead i from list entries [k0, k1): the shared-memory part
-// (k < cap_s), then the part in global memory.
-template <int TERMS, bool ENERGY>
-__device__ __forceinline__ float3 list_forces(int i, int k0, int k1, int cap_s, int npad,
-                                              const uint16_t* slist,
-                                              const uint16_t* __restrict__ glist,
-                                              const float4* sx, const float4* sp0,
-                                              const float4* sp1, uint32_t excl_all,
-                                              const PairConsts& pc, EnergyAcc& ea) {
+// Main force on bead i from the cnt entries of column col, four entries at a
+// time with every load issued before the arithmetic, in list (= increasing
+// j) order.
+template <int CLS, bool ENERGY>
+__device__ __forceinline__ float3 main_list(int i, int col, int cnt, const UnitList& L, const float4* sx,
+                                            const PairParams& P, uint32_t excl_all, const PairConsts& pc,
+                                            EnergyAcc& ea) {
+    float3 f = make_float3(0.f, 0.f, 0.f);
     const float4 xi = sx[i];
-    const float4 p0i = sp0[i];
-    const float4 p1i = (TERMS & kTermLJA) ? sp1[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    float3 fa = make_float3(0.f, 0.f, 0.f);
-    const int ks = min(k1, cap_s);
-    if (k0 < ks) list_range<TERMS, ENERGY>(i, k0, ks, npad, slist, xi, p0i, p1i, sx, sp0, sp1, excl_all, pc, fa, ea);
-    const int kg = max(k0, cap_s);
-    if (kg < k1) list_range<TERMS, ENERGY>(i, kg, k1, npad, glist, xi, p0i, p1i, sx, sp0, sp1, excl_all, pc, fa, ea);
-    return fa;
+    if (CLS == kClassGo) {
+        list_walk(L, col, cnt, [&](uint2 e) {
+            float4 xj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) xj[u] = sx[entry_of(e, u)];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) exv_pair<ENERGY>(xi, xj[u], pc, f, ea);
+        });
+    } else if (CLS == kClassHps) {
+        const float2 lei = P.le[i];
+        list_walk(L, col, cnt, [&](uint2 e) {
+            float4 xj[4];
+            float2 lej[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                xj[u] = sx[entry_of(e, u)];
+                lej[u] = P.le[entry_of(e, u)];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) hps_pair<ENERGY>(xi, xj[u], lei, lej[u], pc, f, ea);
+        });
+    } else {
+        const float4 p0i = P.p0[i], p1i = P.p1[i];
+        list_walk(L, col, cnt, [&](uint2 e) {
+            float4 xj[4], p0j[4], p1j[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int j = (int)(entry_of(e, u) & 2047u);
+                xj[u] = sx[j];
+                p0j[u] = P.p0[j];
+                p1j[u] = P.p1[j];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                general_pair<ENERGY>(xi, xj[u], p0i, p0j[u], p1i, p1j[u], (entry_of(e, u) >> 11) | excl_all, pc, f, ea);
+        });
+    }
+    return f;
 }
 
-// The same sum without a list, for a system whose list overflowed: every
-// j in [j0, j1) in increasing order, the clusters culled by their bounding
+template <bool ENERGY>
+__device__ __forceinline__ float3 charged_list(int i, int col, int cnt, const UnitList& L, const float4* sx,
+                                               const PairParams& P, const PairConsts& pc, EnergyAcc& ea) {
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    const float4 xi = sx[i];
+    const float qk = __fmul_rn(P.q[i], pc.dh_k);
+    list_walk(L, col, cnt, [&](uint2 e) {
+        float4 xj[4];
+        float qj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            xj[u] = sx[entry_of(e, u)];
+            qj[u] = P.q[entry_of(e, u)];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) dh_pair<ENERGY>(xi, xj[u], qk, qj[u], pc, f, ea);
+    });
+    return f;
+}
+
+// The same sums without a list, for a system whose lists overflowed: every
+// j of the range in increasing order, the clusters culled by their bounding
 // boxes at the cutoff.  The nonzero contributions and their order are those
 // of the list walk, so the force is bit-identical to it.
-template <int TERMS, bool LABELS, bool ENERGY>
-__device__ __forceinline__ float3 scan_forces(int i, int j0, int j1, int nt, const float4* sx, const float4* sp0,
-                                              const float4* sp1, const uint32_t* slab, const float4* bc,
-                                              const float4* bh, float cull2, const int32_t* __restrict__ ex_start,
-                                              const int32_t* __restrict__ ex, uint32_t excl_all,
-                                              const PairConsts& pc, EnergyAcc& ea) {
+template <int CLS, bool ENERGY>
+__device__ __forceinline__ float3 main_scan(int i, int j0, int j1, const float4* sx, const PairParams& P,
+                                            const float4* bc, const float4* bh, float cull2,
+                                            const int32_t* __restrict__ ex_start, const int32_t* __restrict__ ex,
+                                            uint32_t excl_all, const PairConsts& pc, EnergyAcc& ea) {
     const float4 xi = sx[i];
-    const float4 p0i = sp0[i];
-    const float4 p1i = (TERMS & kTermLJA) ? sp1[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t labi = LABELS ? slab[i] : 0u;
     const uint32_t present = (uint32_t)pc.terms;
+    const uint32_t drop = CLS == kClassGo ? kTermEXV : kTermLJR;
     int ep = ex_start[i];
     const int e1 = ex_start[i + 1];
     int ej = ep < e1 ? (ex[ep] & 0xFFFFFF) : 0x7FFFFFFF;
-    float3 fa = make_float3(0.f, 0.f, 0.f);
-    for (int J = j0 >> 5; J < nt && J * 32 < j1; ++J) {
-        const float4 c = bc[J], h = bh[J];
-        const float gx = fmaxf(0.f, fabsf(xi.x - c.x) - h.x);
-        const float gy = fmaxf(0.f, fabsf(xi.y - c.y) - h.y);
-        const float gz = fmaxf(0.f, fabsf(xi.z - c.z) - h.z);
-        if (gx * gx + gy * gy + gz * gz >= cull2) continue;
-        const int ja = max(j0, J * 32), jz = min(j1, J * 32 + 32);
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    for (int jb = j0 & ~31; jb < j1; jb += 32) {
+        if (box_far(xi, bc[jb >> 5], bh[jb >> 5], cull2)) continue;
+        const int ja = max(j0, jb), jz = min(j1, jb + 32);
         for (int j = ja; j < jz; ++j) {
             if (j == i) continue;
             uint32_t bits = excl_walk(j, ep, ej, e1, ex);
-            if (LABELS) bits |= label_bits<true>(labi, slab[j], pc);
-            if ((bits & present) == present) continue;
-            pair_accumulate<TERMS, ENERGY>(i, j, xi, sx[j], p0i, p1i, sp0, sp1, bits | excl_all, pc, fa, ea);
+            if (CLS == kClassGeneral) {
+                bits |= label_bits<true>(P.lab[i], P.lab[j], pc);
+                if ((bits & present) == present) continue;
+                general_pair<ENERGY>(xi, sx[j], P.p0[i], P.p0[j], P.p1[i], P.p1[j], bits | excl_all, pc, f, ea);
+            } else {
+                if (bits & drop) continue;
+                if (CLS == kClassGo) exv_pair<ENERGY>(xi, sx[j], pc, f, ea);
+                else hps_pair<ENERGY>(xi, sx[j], P.le[i], P.le[j], pc, f, ea);
+            }
         }
     }
-    return fa;
+    return f;
+}
+
+template <bool ENERGY>
+__device__ __forceinline__ float3 charged_scan(int i, int c0, int c1, const float4* sx, const uint16_t* qidx,
+                                               const PairParams& P, const int32_t* __restrict__ ex_start,
+                                               const int32_t* __restrict__ ex, const PairConsts& pc, EnergyAcc& ea) {
+    const float4 xi = sx[i];
+    const float qk = __fmul_rn(P.q[i], pc.dh_k);
+    int ep = ex_start[i];
+    const int e1 = ex_start[i + 1];
+    int ej = ep < e1 ? (ex[ep] & 0xFFFFFF) : 0x7FFFFFFF;
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    for (int c = c0; c < c1; ++c) {
+        const int j = qidx[c];
+        if (j == i || (excl_walk(j, ep, ej, e1, ex) & kTermDH)) continue;
+        dh_pair<ENERGY>(xi, sx[j], qk, P.q[j], pc, f, ea);
+    }
+    return f;
 }
 
 // One claimed system (order entry q, slot `slot`) advanced by a group of GT
 // threads (gtid = 0..GT-1) whose barrier is `bar` (0: the whole CTA), in
 // the group's shared memory [gsmem, gsmem + gsmem_bytes), with the group's
 // shared words (s_move[2], s_overflow, s_bad, s_energy[kNumSlots]).
-template <int GT, int TERMS, bool LABELS, bool ENERGY, bool INTEGRATE>
+template <int GT, int MODE, bool ENERGY, bool INTEGRATE>
 __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, int gtid, int bar,
                                            unsigned char* gsmem, size_t gsmem_bytes, int* s_move,
                                            int* s_overflow, int* s_bad, double* s_energy, int* s_item) {
@@ -610,39 +860,55 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     const float4* gp1 = reinterpret_cast<const float4*>(blob + R.off_p1);
     const uint32_t* glab = reinterpret_cast<const uint32_t*>(blob + R.off_lab);
     const float* ginvm = reinterpret_cast<const float*>(blob + R.off_invm);
+    const int cls = MODE == kClassGo ? kClassGo : R.cls;
+    const bool plain_cls = MODE != kClassGeneral || cls != kClassGeneral;  // Go or Hps
+    const int S = pair_split(n, kSplitUnits), lg = __ffs(S) - 1;
+    const int nq = R.nq, Sq = pair_split(nq, kSplitCharged), lgq = __ffs(Sq) - 1;
+    UnitList lm, lq;
+    lm.cols = list_columns(n, S);
+    lq.cols = list_columns(nq, Sq);
     // ---- shared-memory layout of this system, arrays of stride ns ----
-    // Positions are float-float: hi parts in sx (pair arithmetic), lo
-    // parts in sxl; x = hi + lo carries ~48 significant bits.  fp / fb:
-    // each bead's pair and bonded force of the current step.
+    // Positions are float-float: hi parts in sx (pair arithmetic; .w holds
+    // the Go radius or half the Hps sigma, bead ns is a dummy far away), lo
+    // parts in sxl; x = hi + lo carries ~48 significant bits.  fp / fb / fq:
+    // each bead's pair, bonded and Debye-Hueckel force of the current step
+    // (General: fp holds every pair term).
     const int ns = npad;
-    float* fp = reinterpret_cast<float*>(gsmem);
-    float* fb = reinterpret_cast<float*>(gsmem + 12 * (size_t)ns);
-    float4* sx = reinterpret_cast<float4*>(gsmem + 24 * (size_t)ns);
-    float4* sp0 = reinterpret_cast<float4*>(gsmem + 40 * (size_t)ns);
-    float* sxl = reinterpret_cast<float*>(gsmem + 56 * (size_t)ns);
-    float* sv = reinterpret_cast<float*>(gsmem + 68 * (size_t)ns);
-    float* sim = reinterpret_cast<float*>(gsmem + 80 * (size_t)ns);
-    float* sref = reinterpret_cast<float*>(gsmem + 84 * (size_t)ns);
-    uint16_t* scnt = reinterpret_cast<uint16_t*>(gsmem + 96 * (size_t)ns);
-    uint16_t* bord = reinterpret_cast<uint16_t*>(gsmem + 98 * (size_t)ns);
-    size_t off = (size_t)kBeadBytes * ns;
-    float4* sp1 = nullptr;
+    size_t off = 0;
+    auto carve = [&](size_t bytes) {
+        unsigned char* p = gsmem + off;
+        off += bytes;
+        return p;
+    };
+    float4* sx = reinterpret_cast<float4*>(carve(16 * (size_t)(ns + 1)));
+    float* fp = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+    float* fb = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+    float* sxl = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+    float* sv = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+    float* sim = reinterpret_cast<float*>(carve(4 * (size_t)ns));
+    float* sref = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+    float4 *sp0 = nullptr, *sp1 = nullptr;
     uint32_t* slab = nullptr;
-    if ((TERMS & kTermLJA) || LABELS) {
-        sp1 = reinterpret_cast<float4*>(gsmem + off);
-        slab = reinterpret_cast<uint32_t*>(gsmem + off + 16 * (size_t)ns);
-        off += 20 * (size_t)ns;
+    float *fq = nullptr, *sq = nullptr;
+    float2* sle = nullptr;
+    if (plain_cls) {
+        fq = reinterpret_cast<float*>(carve(12 * (size_t)ns));
+        sq = reinterpret_cast<float*>(carve(4 * (size_t)ns));
+        if (MODE != kClassGo && cls == kClassHps) sle = reinterpret_cast<float2*>(carve(8 * (size_t)ns));
+    } else {
+        sp0 = reinterpret_cast<float4*>(carve(16 * (size_t)ns));
+        sp1 = reinterpret_cast<float4*>(carve(16 * (size_t)ns));
+        slab = reinterpret_cast<uint32_t*>(carve(4 * (size_t)ns));
     }
-    float4* bc = reinterpret_cast<float4*>(gsmem + off);
-    float4* bh = bc + nt;
-    off += 32 * (size_t)nt;
-    float3* carry = reinterpret_cast<float3*>(gsmem + off);
-    off += 36 * (size_t)nt;
+    float4* bc = reinterpret_cast<float4*>(carve(16 * (size_t)nt));
+    float4* bh = reinterpret_cast<float4*>(carve(16 * (size_t)nt));
+    float3* carry = reinterpret_cast<float3*>(carve(36 * (size_t)nt));
+    int* hist = reinterpret_cast<int*>(carve(4 * kSortBuckets));
+    uint16_t* bord = reinterpret_cast<uint16_t*>(carve(2 * (size_t)ns));
+    uint16_t* ucnt = reinterpret_cast<uint16_t*>(carve(2 * (size_t)lm.cols));
+    uint16_t* qidx = reinterpret_cast<uint16_t*>(carve(2 * (size_t)((nq + 31) & ~31)));
+    uint16_t* qcnt = reinterpret_cast<uint16_t*>(carve(2 * (size_t)lq.cols));
     off = (off + 15) & ~(size_t)15;
-    uint16_t* sseg = reinterpret_cast<uint16_t*>(gsmem + off);
-    off += 2 * kMaxUnits;
-    int* hist = reinterpret_cast<int*>(gsmem + off);
-    off += 4 * kSortBuckets;
     // bonded records and tables: staged in shared memory when they fit,
     // read from the blob otherwise
     const unsigned char* gbonded = blob + R.off_bonded;
@@ -664,15 +930,20 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     B.cd = reinterpret_cast<const uint16_t*>(bsrc + R.rcd);
     B.gs = reinterpret_cast<const uint16_t*>(bsrc + R.rgs);
     B.gl = reinterpret_cast<const uint32_t*>(bsrc + R.rgl);
-    uint16_t* slist = reinterpret_cast<uint16_t*>(gsmem + off);
+    // the lists' shared-memory part: the charged lists first (they are
+    // short), at most half of what is left, then the main lists
     const size_t list_bytes = gsmem_bytes > off ? gsmem_bytes - off : 0;
+    lq.cap = R.maxq;
+    lq.cap_s = lq.cols ? min(lq.cap, (int)(list_bytes / 2 / (2 * (size_t)lq.cols)) & ~3) : 0;
+    lq.s = reinterpret_cast<uint16_t*>(gsmem + off);
+    const size_t q_bytes = 2 * (size_t)lq.cap_s * lq.cols;
+    lm.cap = R.maxn;
+    lm.cap_s = min(lm.cap, (int)((list_bytes - q_bytes) / (2 * (size_t)lm.cols)) & ~3);
+    lm.s = reinterpret_cast<uint16_t*>(gsmem + off + q_bytes);
+    lm.g = a.lists + R.list_off;
+    lq.g = lm.g + (size_t)lm.cap * lm.cols;
     const int32_t* ex_start = reinterpret_cast<const int32_t*>(blob + R.off_ex_start);
     const int32_t* exl = reinterpret_cast<const int32_t*>(blob + R.off_ex);
-    uint16_t* glist = a.lists + R.list_off;
-    const int maxn = R.maxn;
-    // entries per bead kept in shared memory (multiple of 4)
-    const int cap_s = min(maxn, (int)(list_bytes / (2 * (size_t)npad)) & ~3);
-    const int S = pair_split(n);
     const unsigned long long step0 = R.steps_done;
     int K = 1;
     if (INTEGRATE) {
@@ -685,7 +956,11 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     if (!(slots_en & (1u << kSlotDH))) excl_all |= kTermDH;
     if (!(slots_en & (1u << kSlotLJR))) excl_all |= kTermLJR;
     if (!(slots_en & (1u << kSlotLJA))) excl_all |= kTermLJA;
-    const bool pairs_on = (pc.terms & ~excl_all) != 0;
+    // main and charged passes that run; an excluded Lennard-Jones term of an
+    // Hps system enters with zero epsilon
+    const bool main_on = plain_cls ? (pc.terms & ~excl_all & ~kTermDH) != 0 : (pc.terms & ~excl_all) != 0;
+    const bool dh_on = plain_cls && nq > 0 && (pc.terms & ~excl_all & kTermDH) != 0;
+    const bool pairs_on = main_on || dh_on;
 
     // ---- load ----
     for (int b = gtid; b < npad; b += GT) {
@@ -693,51 +968,63 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
             const double px = a.x[boff + b], py = a.y[boff + b], pz = a.z[boff + b];
             const float hx = __double2float_rn(px), hy = __double2float_rn(py),
                         hz = __double2float_rn(pz);
-            sx[b] = make_float4(hx, hy, hz, 0.f);
+            const float4 p0 = gp0[b];
+            sx[b] = make_float4(hx, hy, hz, MODE != kClassGo && cls == kClassHps ? 0.5f * p0.w : p0.x);
             sxl[b] = __double2float_rn(px - (double)hx);
             sxl[ns + b] = __double2float_rn(py - (double)hy);
             sxl[2 * ns + b] = __double2float_rn(pz - (double)hz);
-            sp0[b] = gp0[b];
             sv[b] = a.vx[boff + b];
             sv[ns + b] = a.vy[boff + b];
             sv[2 * ns + b] = a.vz[boff + b];
             sim[b] = ginvm[b];
-            if ((TERMS & kTermLJA) || LABELS) {
+            bord[b] = a.bead_order[boff + b];
+            if (plain_cls) sq[b] = p0.y;
+            if (MODE != kClassGo && cls == kClassHps)
+                sle[b] = make_float2(excl_all & kTermLJR ? 0.f : 0.5f * p0.z, excl_all & kTermLJA ? 0.f : 0.5f * gp1[b].x);
+            if (!plain_cls) {
+                sp0[b] = p0;
                 sp1[b] = gp1[b];
                 slab[b] = glab[b];
             }
         } else {
             sx[b] = make_float4(nan, nan, nan, 0.f);
-            sp0[b] = make_float4(0.f, 0.f, 0.f, 0.f);
             sim[b] = 0.f;
-            if ((TERMS & kTermLJA) || LABELS) {
-                sp1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!plain_cls) {
+                sp0[b] = sp1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
                 slab[b] = 0xffffffffu;
             }
         }
+        // uncharged beads keep a zero Debye-Hueckel force, and every bead a
+        // zero pair force when no pair pass runs
+        for (int c = 0; c < 3; ++c) {
+            fp[c * ns + b] = 0.f;
+            if (plain_cls) fq[c * ns + b] = 0.f;
+        }
     }
+    if (gtid == 0) sx[ns] = make_float4(1e15f, 1e15f, 1e15f, 0.f);
+    const uint16_t* gqidx = reinterpret_cast<const uint16_t*>(blob + R.off_qidx);
+    for (int c = gtid; c < nq; c += GT) qidx[c] = gqidx[c];
     if (bonded_smem) {
         const uint4* src = reinterpret_cast<const uint4*>(gbonded);
         uint4* dst = reinterpret_cast<uint4*>(sbonded);
         for (int q = gtid; q < R.bonded_bytes / 16; q += GT) dst[q] = src[q];
     }
     for (int k = gtid; k < kSortBuckets; k += GT) hist[k] = 0;
-    for (int b = gtid; b < n; b += GT) bord[b] = (uint16_t)b;  // until the first list build
     if (gtid == 0) *s_item = 0;
     bar_sync(bar, GT);
-    for (int I = gwarp; I < nt; I += NWG) cluster_bbox(I, n, sx, bc, bh, lane);
-    bar_sync(bar, GT);
 
-    // list cutoff = largest pair cutoff + skin; the scan culls at the
-    // cutoff (with a margin for the FP32 box arithmetic)
-    const float rc = sqrtf(pc.list_rc2);
-    const float lcut = (rc + R.skin) * 1.0001f;
-    const float lcut2 = lcut * lcut;
-    const float tcut = rc * 1.0001f + 1e-4f;
+    // list cutoff = pair cutoff + skin; the scan culls at the cutoff (with a
+    // margin for the FP32 box arithmetic)
+    const float lcut = (R.main_rc + R.skin) * 1.0001f;
+    const float lcut2 = main_on ? lcut * lcut : -1.f;
+    const float qcut = (R.dh_rc + R.skin) * 1.0001f;
+    const float qcut2 = qcut * qcut;
+    const float tcut = R.main_rc * 1.0001f + 1e-4f;
     const float tcut2 = tcut * tcut;
     const float half_skin2 = 0.25f * R.skin * R.skin;
     bool use_scan = false;
     bool need_build = pairs_on;
+    const PairParams pp{sp0, sp1, slab, sle, sq};
     int builds = 0;
     int st_done = 0;
     EnergyAcc ea;
@@ -745,31 +1032,59 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
 
     for (int st = 0; st < K; ++st) {
         if (need_build && !use_scan) {
-            // fb is free until the bonded terms of this step: sort scratch
-            build_lists<LABELS>(n, nt, npad, maxn, cap_s, lcut2, sx, slab, bc, bh, ex_start, exl,
-                                pc, slist, glist, scnt, sref, ns, gtid, GT, S, sseg,
-                                s_overflow, bord, hist, reinterpret_cast<uint32_t*>(fb), bar);
+            // fp and fb are free until this step's forces: scratch of the
+            // sort, and the beads' places in the pass order.  The bounding
+            // boxes cull the build (and the scan) only, so they are formed
+            // here and not with every update.
+            uint16_t* pos = reinterpret_cast<uint16_t*>(fb);
+            if (builds > 0 && builds % kSortBuilds == 0)
+                sort_beads(n, lg, ucnt, bord, hist, reinterpret_cast<uint32_t*>(fb), reinterpret_cast<uint16_t*>(fp), gtid,
+                           GT, bar);
+            for (int I = gwarp; I < nt; I += NWG) cluster_bbox(I, n, sx, bc, bh, lane);
+            for (int p = gtid; p < n; p += GT) pos[bord[p]] = (uint16_t)p;
+            for (int b = gtid; b < n; b += GT) {
+                const float4 h = sx[b];
+                sref[b] = h.x;
+                sref[ns + b] = h.y;
+                sref[2 * ns + b] = h.z;
+            }
+            bar_sync(bar, GT);
+            if (cls == kClassGo)
+                build_main<kClassGo>(n, lg, lcut2, sx, slab, bc, bh, ex_start, exl, pc, lm, pos, ucnt, ns, gtid, GT,
+                                     s_overflow);
+            else if (MODE != kClassGo && cls == kClassHps)
+                build_main<kClassHps>(n, lg, lcut2, sx, slab, bc, bh, ex_start, exl, pc, lm, pos, ucnt, ns, gtid, GT,
+                                      s_overflow);
+            else if (MODE == kClassGeneral)
+                build_main<kClassGeneral>(n, lg, lcut2, sx, slab, bc, bh, ex_start, exl, pc, lm, pos, ucnt, ns, gtid, GT,
+                                          s_overflow);
+            if (dh_on) build_charged(nq, lgq, qcut2, sx, qidx, ex_start, exl, lq, qcnt, ns, gtid, GT, s_overflow);
             ++builds;
             bar_sync(bar, GT);
             use_scan = *s_overflow != 0;
+            if (!main_on)  // the scratch lay in the pair forces
+                for (int b = gtid; b < 3 * ns; b += GT) fp[b] = 0.f;
+        } else if (use_scan) {
+            for (int I = gwarp; I < nt; I += NWG) cluster_bbox(I, n, sx, bc, bh, lane);
+            bar_sync(bar, GT);
         }
         const unsigned long long step = step0 + (unsigned long long)st;
         // ---- forces: warps claim work items from the group's counter,
         // the bonded clusters first, then the pair passes, longest first
         // (claiming the longest passes before the bonded clusters measured
-        // slower).  Pair pass p covers units u = 32 p + lane
-        // of the sorted beads: the S units of bead bord[u / S] are adjacent
-        // lanes (sub-lane u % S sums the list entries whose j lies in its
-        // j-range); their partial sums meet in a fixed butterfly and the
-        // first sub-lane stores the bead's pair force.  Every bead's sum is
-        // the same whichever warp and lanes compute it. ----
-        const int n_pass = pairs_on ? (n * S + 31) >> 5 : 0;
-        const int lg_s = __ffs(S) - 1;
+        // slower), then the charged passes.  Pair pass p covers units
+        // u = 32 p + lane of the sorted beads: the S units of bead
+        // bord[u / S] are adjacent lanes (sub-lane u % S sums the entries
+        // whose j lies in its j-range); their partial sums meet in a fixed
+        // butterfly and the first sub-lane stores the bead's pair force.
+        // Every bead's sum is the same whichever warp and lanes compute it. ----
+        const int n_main = main_on ? ((n << lg) + 31) >> 5 : 0;
+        const int n_items = nt + n_main + (dh_on ? ((nq << lgq) + 31) >> 5 : 0);
         while (true) {
             int it = 0;
             if (lane == 0) it = atomicAdd(s_item, 1);
             it = __shfl_sync(kFull, it, 0);
-            if (it >= nt + n_pass) break;
+            if (it >= n_items) break;
             if (it < nt) {
                 const float3 f = bonded_cluster<ENERGY>(B, it, n, lane, sx, sxl, ns, slots_en, carry, ea);
                 const int b = it * 32 + lane;
@@ -780,38 +1095,59 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
                 }
                 continue;
             }
-            const int u = ((it - nt) << 5) + lane;
-            const int sb = u >> lg_s, sr = u & (S - 1);
-            const int i = sb < n ? (int)bord[sb] : n;
             float3 fi = make_float3(0.f, 0.f, 0.f);
-            if (i < n) {
+            const bool charged = it >= nt + n_main;
+            const int u = ((it - nt - (charged ? n_main : 0)) << 5) + lane;
+            const int split = charged ? Sq : S;
+            int i = n;
+            if (charged) {
+                if (u < nq << lgq) {
+                    i = (int)qidx[u >> lgq];
+                    if (!use_scan) {
+                        fi = charged_list<ENERGY>(i, u, (int)qcnt[u], lq, sx, pp, pc, ea);
+                    } else {
+                        const int s = u & (Sq - 1);
+                        fi = charged_scan<ENERGY>(i, (s * nq) >> lgq, ((s + 1) * nq) >> lgq, sx, qidx, pp, ex_start, exl,
+                                                  pc, ea);
+                    }
+                }
+            } else if (u < n << lg) {
+                i = (int)bord[u >> lg];
                 if (!use_scan) {
-                    const int k0 = S > 1 ? (int)sseg[i * S + sr] : 0;
-                    const int k1 = sr == S - 1 ? (int)scnt[i] : (int)sseg[i * S + sr + 1];
-                    fi = list_forces<TERMS, ENERGY>(i, k0, k1, cap_s, npad, slist, glist, sx, sp0, sp1,
-                                                    excl_all, pc, ea);
+                    const int cnt = (int)ucnt[u];
+                    if (cls == kClassGo) fi = main_list<kClassGo, ENERGY>(i, u, cnt, lm, sx, pp, excl_all, pc, ea);
+                    else if (MODE != kClassGo && cls == kClassHps)
+                        fi = main_list<kClassHps, ENERGY>(i, u, cnt, lm, sx, pp, excl_all, pc, ea);
+                    else if (MODE == kClassGeneral)
+                        fi = main_list<kClassGeneral, ENERGY>(i, u, cnt, lm, sx, pp, excl_all, pc, ea);
                 } else {
-                    const int j0 = (sr * n) / S, j1 = sr == S - 1 ? n : ((sr + 1) * n) / S;
-                    fi = scan_forces<TERMS, LABELS, ENERGY>(i, j0, j1, nt, sx, sp0, sp1, slab, bc, bh,
-                                                            tcut2, ex_start, exl, excl_all, pc, ea);
+                    const int s = u & (S - 1), j0 = (s * n) >> lg, j1 = ((s + 1) * n) >> lg;
+                    if (cls == kClassGo)
+                        fi = main_scan<kClassGo, ENERGY>(i, j0, j1, sx, pp, bc, bh, tcut2, ex_start, exl, excl_all, pc, ea);
+                    else if (MODE != kClassGo && cls == kClassHps)
+                        fi = main_scan<kClassHps, ENERGY>(i, j0, j1, sx, pp, bc, bh, tcut2, ex_start, exl, excl_all, pc,
+                                                          ea);
+                    else if (MODE == kClassGeneral)
+                        fi = main_scan<kClassGeneral, ENERGY>(i, j0, j1, sx, pp, bc, bh, tcut2, ex_start, exl, excl_all,
+                                                              pc, ea);
                 }
             }
-            for (int o = 1; o < S; o <<= 1) {
+            for (int o = 1; o < split; o <<= 1) {
                 fi.x += __shfl_xor_sync(kFull, fi.x, o);
                 fi.y += __shfl_xor_sync(kFull, fi.y, o);
                 fi.z += __shfl_xor_sync(kFull, fi.z, o);
             }
-            if (i < n && sr == 0) {
-                fp[i] = fi.x;
-                fp[ns + i] = fi.y;
-                fp[2 * ns + i] = fi.z;
+            if (i < n && (u & (split - 1)) == 0) {
+                float* out = charged ? fq : fp;
+                out[i] = fi.x;
+                out[ns + i] = fi.y;
+                out[2 * ns + i] = fi.z;
             }
         }
         bar_sync(bar, GT);
         if (gtid == 0) *s_item = 0;  // read again only after the next barrier
         if (!INTEGRATE) break;
-        // ---- Langevin update, bounding boxes, displacement and
-        // blow-up checks; bead b = I * 32 + lane of cluster I = gwarp +
+        // ---- Langevin update, displacement and blow-up checks; bead b = I * 32 + lane of cluster I = gwarp +
         // c * NWG ----
         const int mv = st & 1;
 #pragma unroll 4
@@ -821,11 +1157,11 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
             const int b = I * 32 + lane;
             bool moved = false, bad = false;
             if (b < n) {
-                float fx = fb[b], fy = fb[ns + b], fz = fb[2 * ns + b];
-                if (pairs_on) {
-                    fx = fp[b] + fx;
-                    fy = fp[ns + b] + fy;
-                    fz = fp[2 * ns + b] + fz;
+                float fx = fp[b] + fb[b], fy = fp[ns + b] + fb[ns + b], fz = fp[2 * ns + b] + fb[2 * ns + b];
+                if (plain_cls) {
+                    fx += fq[b];
+                    fy += fq[ns + b];
+                    fz += fq[2 * ns + b];
                 }
                 if (lane < 3 && I > 0) {
                     const float3 cin = carry[3 * (I - 1) + lane];
@@ -857,18 +1193,21 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
             }
             if (__any_sync(kFull, moved) && lane == 0) atomicOr(&s_move[mv], 1);
             if (__any_sync(kFull, bad) && lane == 0) atomicOr(s_bad, 1);
-            __syncwarp();
-            cluster_bbox(I, n, sx, bc, bh, lane);
         }
         bar_sync(bar, GT);
         st_done = st + 1;
         if (*s_bad) break;  // the system blew up this step: stop advancing it
-        need_build = s_move[mv] != 0;
+        need_build = pairs_on && s_move[mv] != 0;
         if (gtid == 0) s_move[mv ^ 1] = 0;
     }
 
     // ---- write back ----
     if (INTEGRATE) {
+        if (builds > 0) {  // the pass order of the next launch
+            sort_beads(n, lg, ucnt, bord, hist, reinterpret_cast<uint32_t*>(fb), reinterpret_cast<uint16_t*>(fp), gtid, GT,
+                       bar);
+            for (int p = gtid; p < n; p += GT) a.bead_order[boff + p] = bord[p];
+        }
         for (int b = gtid; b < n; b += GT) {
             const float4 h = sx[b];
             a.x[boff + b] = (double)h.x + (double)sxl[b];
@@ -887,11 +1226,11 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     } else {
         bool bad = false;
         for (int b = gtid; b < n; b += GT) {
-            float fx = fb[b], fy = fb[ns + b], fz = fb[2 * ns + b];
-            if (pairs_on) {
-                fx = fp[b] + fx;
-                fy = fp[ns + b] + fy;
-                fz = fp[2 * ns + b] + fz;
+            float fx = fp[b] + fb[b], fy = fp[ns + b] + fb[ns + b], fz = fp[2 * ns + b] + fb[2 * ns + b];
+            if (plain_cls) {
+                fx += fq[b];
+                fy += fq[ns + b];
+                fz += fq[2 * ns + b];
             }
             const int I = b >> 5, l = b & 31;
             if (l < 3 && I > 0) {
@@ -923,7 +1262,7 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     }
 }
 
-template <int THREADS, int TERMS, bool LABELS, bool ENERGY, bool INTEGRATE>
+template <int THREADS, int MODE, bool ENERGY, bool INTEGRATE>
 __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     // per-group state (group 0 only until the split)
@@ -965,8 +1304,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
             split_q = q;
             break;
         }
-        run_system<THREADS, TERMS, LABELS, ENERGY, INTEGRATE>(a, q, slot, tid, 0, smem, a.smem_bytes, s_move[0],
-                                                              &s_overflow[0], &s_bad[0], s_energy[0], &s_item[0]);
+        run_system<THREADS, MODE, ENERGY, INTEGRATE>(a, q, slot, tid, 0, smem, a.smem_bytes, s_move[0], &s_overflow[0],
+                                                     &s_bad[0], s_energy[0], &s_item[0]);
         __syncthreads();
     }
 
@@ -1002,8 +1341,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
             bar_sync(1 + g, GT);
             continue;
         }
-        run_system<GT, TERMS, LABELS, ENERGY, INTEGRATE>(a, q, slot, gtid, 1 + g, gsmem, half, s_move[g],
-                                                         &s_overflow[g], &s_bad[g], s_energy[g], &s_item[g]);
+        run_system<GT, MODE, ENERGY, INTEGRATE>(a, q, slot, gtid, 1 + g, gsmem, half, s_move[g], &s_overflow[g],
+                                                &s_bad[g], s_energy[g], &s_item[g]);
         bar_sync(1 + g, GT);
     }
 }
@@ -1077,33 +1416,43 @@ void launch_persistent(Fn fn, int threads, BatchArgs a, int max_grid, size_t sme
     OCM_CK(cudaGetLastError());
 }
 
-template <int THREADS, int TERMS, bool LABELS>
-void launch_batch_t(const BatchArgs& a, int max_grid, size_t smem, cudaStream_t s, bool integrate,
-                    bool energy, int num_sms, size_t lkib) {
-    if (integrate)
-        launch_persistent(k_batch<THREADS, TERMS, LABELS, false, true>, THREADS, a, max_grid, smem, s, num_sms, lkib);
-    else if (energy)
-        launch_persistent(k_batch<THREADS, TERMS, LABELS, true, false>, THREADS, a, max_grid, smem, s, num_sms, lkib);
-    else
-        launch_persistent(k_batch<THREADS, TERMS, LABELS, false, false>, THREADS, a, max_grid, smem, s, num_sms, lkib);
+template <int THREADS, int MODE>
+void launch_batch_t(const BatchArgs& a, int max_grid, size_t smem, cudaStream_t s, bool integrate, int num_sms,
+                    size_t lkib) {
+    if (integrate) launch_persistent(k_batch<THREADS, MODE, false, true>, THREADS, a, max_grid, smem, s, num_sms, lkib);
+    else launch_persistent(k_batch<THREADS, MODE, true, false>, THREADS, a, max_grid, smem, s, num_sms, lkib);
 }
 
-template <int TERMS, bool LABELS>
-void launch_batch_threads(int threads, const BatchArgs& a, int grid, size_t smem, cudaStream_t s,
-                          bool integrate, bool energy, int num_sms, size_t lkib) {
+template <int MODE>
+void launch_batch_threads(int threads, const BatchArgs& a, int grid, size_t smem, cudaStream_t s, bool integrate,
+                          int num_sms, size_t lkib) {
     switch (threads) {
-        case 256: launch_batch_t<256, TERMS, LABELS>(a, grid, smem, s, integrate, energy, num_sms, lkib); break;
-        case 512: launch_batch_t<512, TERMS, LABELS>(a, grid, smem, s, integrate, energy, num_sms, lkib); break;
-        default: launch_batch_t<1024, TERMS, LABELS>(a, grid, smem, s, integrate, energy, num_sms, lkib); break;
+        case 256: launch_batch_t<256, MODE>(a, grid, smem, s, integrate, num_sms, lkib); break;
+        case 512: launch_batch_t<512, MODE>(a, grid, smem, s, integrate, num_sms, lkib); break;
+        default: launch_batch_t<1024, MODE>(a, grid, smem, s, integrate, num_sms, lkib); break;
+    }
+}
+
+// The kernel for the classes up to `cls` (kClassGeneral runs them all): a
+// launch of Go systems alone does not carry the other classes' registers.
+// integrate: MD steps; otherwise one evaluation of forces and energies.
+void launch_batch(int cls, int threads, const BatchArgs& a, int grid, size_t smem, cudaStream_t s, bool integrate,
+                  int num_sms, size_t lkib) {
+    switch (cls) {
+        case kClassGo: launch_batch_threads<kClassGo>(threads, a, grid, smem, s, integrate, num_sms, lkib); break;
+        case kClassHps: launch_batch_threads<kClassHps>(threads, a, grid, smem, s, integrate, num_sms, lkib); break;
+        default: launch_batch_threads<kClassGeneral>(threads, a, grid, smem, s, integrate, num_sms, lkib); break;
     }
 }
 
 int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 // The bonded terms of one system in kernel order.  A term is chain-local
-// when its beads are consecutive chain positions (bond b, b+1; angle b..b+2;
-// dihedral b..b+3, either direction; angles and dihedrals are reversed to
-// increasing order, which leaves the angle and the torsion unchanged).
+// when its beads are within four consecutive chain positions (bond from b to
+// b+1, b+2 or b+3, the reach of the AICG2+ local contacts, which as gather
+// entries were evaluated by both of their beads; angle b..b+2; dihedral
+// b..b+3, either direction; angles and dihedrals are reversed to increasing
+// order, which leaves the angle and the torsion unchanged).
 // Chain-local terms come first, sorted by their first bead (stable, so
 // terms on the same beads keep their order), with per-bead start indices;
 // every other term is listed in the gather entries of each of its beads
@@ -1127,7 +1476,7 @@ BondedPlan plan_bonded(const CompiledSystem& c) {
     std::vector<std::pair<int64_t, DihedralTerm>> chd;
     for (BondTerm t : c.bonds) {
         if (t.i > t.j) std::swap(t.i, t.j);
-        if (t.j == t.i + 1) chb.emplace_back(t.i, t);
+        if (t.j <= t.i + 3) chb.emplace_back(t.i, t);
         else ob.push_back(t);
     }
     for (AngleTerm t : c.angles) {
@@ -1197,7 +1546,7 @@ BondedPlan plan_bonded(const CompiledSystem& c) {
 
 struct BlobLayout {
     int64_t size = 0;
-    int off_p0, off_p1, off_lab, off_invm, off_ex_start, off_ex;
+    int off_p0, off_p1, off_lab, off_invm, off_ex_start, off_ex, off_qidx;
     int off_bonded, bonded_bytes, rb_p, rb_ij, ra_ij, ra_k, rd, rgd, rfla, rfld;
     int rcb, rca, rcd, rgs, rgl;
 };
@@ -1240,32 +1589,76 @@ BlobLayout blob_layout(const CompiledSystem& c, const BondedPlan& P) {
     L.bonded_bytes = (int)(o - L.off_bonded);
     L.off_ex_start = take(4 * (n + 1));
     L.off_ex = take(4 * (int64_t)c.ex_j.size());
+    L.off_qidx = take(2 * n);
     L.size = align_up(o, 256);
     return L;
 }
 
 constexpr float kBatchSkin = 0.3f;  // nm
 
-// Entries per bead of a system's neighbour list: the largest count within
-// the list cutoff at admission, with head-room for compaction.
-int initial_list_capacity(const CompiledSystem& c, const double* pos) {
-    const int64_t n = c.n;
-    if (c.pc.terms == 0) return 1;
-    const double cut = std::sqrt((double)c.pc.list_rc2) + kBatchSkin;
-    const double cut2 = cut * cut;
-    int mx = 0;
-    for (int64_t i = 0; i < n; ++i) {
-        int cnt = 0;
-        for (int64_t j = 0; j < n; ++j) {
-            if (j == i) continue;
-            const double dx = pos[3 * j] - pos[3 * i], dy = pos[3 * j + 1] - pos[3 * i + 1],
-                         dz = pos[3 * j + 2] - pos[3 * i + 2];
-            cnt += dx * dx + dy * dy + dz * dz < cut2;
-        }
-        mx = std::max(mx, cnt);
+// Class of a system and the cutoffs of its two lists.
+struct PairPlan {
+    int cls = kClassGeneral;
+    double main_rc = 0, dh_rc = 0;  // 0: no such pairs
+    std::vector<uint16_t> charged;  // Go and Hps: charged beads in increasing order
+};
+
+PairPlan plan_pairs(const CompiledSystem& c) {
+    PairPlan P;
+    const PairConsts& pc = c.pc;
+    bool same = true;  // the two Lennard-Jones terms exclude the same pairs
+    for (uint8_t b : c.ex_bits) same = same && ((b & kTermLJR) != 0) == ((b & kTermLJA) != 0);
+    if (!pc.uses_labels && (pc.terms & ~(kTermEXV | kTermDH)) == 0) P.cls = kClassGo;
+    else if (!pc.uses_labels && (pc.terms & ~kTermDH) == (kTermLJR | kTermLJA) && c.lj_same_sigma && !pc.ljr_geometric &&
+             pc.ljr_rc2 == pc.lja_rc2 && same)
+        P.cls = kClassHps;
+    if (P.cls == kClassGeneral) {
+        P.main_rc = pc.terms ? std::sqrt((double)pc.list_rc2) : 0.0;
+        return P;
     }
+    if (pc.terms & kTermEXV) P.main_rc = std::sqrt((double)pc.exv_rc2);
+    if (P.cls == kClassHps) P.main_rc = std::sqrt((double)pc.lja_rc2);
+    if (pc.terms & kTermDH) {
+        P.dh_rc = std::sqrt((double)pc.dh_rc2);
+        for (int64_t i = 0; i < c.n; ++i)
+            if (c.p0[4 * i + 1] != 0.f) P.charged.push_back((uint16_t)i);
+    }
+    return P;
+}
+
+// Entries per unit of the lists over the m beads idx (or all of them), each
+// bead's partners split into S ranges: the largest count within the list
+// cutoff at admission, with head-room for compaction; at most the range.
+int unit_capacity_limit(int64_t m, int S) { return (int)align_up(std::max<int64_t>(1, (m + S - 1) / S), 4); }
+
+int initial_list_capacity(int64_t m, const uint16_t* idx, int S, double rc, const double* pos) {
+    if (rc <= 0 || m == 0) return 4;
+    const double cut = rc + kBatchSkin, cut2 = cut * cut;
+    std::vector<double> x(m), y(m), z(m);
+    for (int64_t k = 0; k < m; ++k) {
+        const int64_t i = idx ? idx[k] : k;
+        x[k] = pos[3 * i];
+        y[k] = pos[3 * i + 1];
+        z[k] = pos[3 * i + 2];
+    }
+    int mx = 0;
+    for (int64_t i = 0; i < m; ++i)
+        for (int s = 0; s < S; ++s) {
+            int cnt = 0;
+            for (int64_t j = s * m / S; j < (s + 1) * m / S; ++j) {
+                const double dx = x[j] - x[i], dy = y[j] - y[i], dz = z[j] - z[i];
+                cnt += dx * dx + dy * dy + dz * dz < cut2;
+            }
+            mx = std::max(mx, cnt);
+        }
     const int cap = (int)std::ceil(1.25 * mx) + 16;
-    return (int)std::min<int64_t>(std::max<int64_t>(1, n - 1), align_up(cap, 4));
+    return std::min((int)align_up(cap, 4), unit_capacity_limit(m, S));
+}
+
+// Entries that a system's two lists take, main first.
+int64_t list_entries(const BatchSys& R) {
+    return (int64_t)R.maxn * list_columns(R.n, pair_split(R.n, kSplitUnits)) +
+           (int64_t)R.maxq * list_columns(R.nq, pair_split(R.nq, kSplitCharged));
 }
 
 void check_batchable(const CompiledSystem& c, int nmax) {
@@ -1328,7 +1721,7 @@ BatchEngine::BatchEngine(int device, int64_t max_systems, int64_t max_beads, int
     OCM_CK(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device));
     int optin = 0;
     OCM_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    if ((int64_t)smem_bytes(nmax_, false) > optin)
+    if ((int64_t)smem_bytes(nmax_, kClassGo) > optin)
         throw Error(6, "[error] per-system bead limit does not fit in shared memory");
     OCM_CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     OCM_CK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
@@ -1346,9 +1739,12 @@ BatchEngine::BatchEngine(int device, int64_t max_systems, int64_t max_beads, int
     x_.alloc(max_beads); y_.alloc(max_beads); z_.alloc(max_beads);
     vx_.alloc(max_beads); vy_.alloc(max_beads); vz_.alloc(max_beads);
     blob_dev_.alloc(blob_cap);
-    const int64_t list_cap = max_beads * 256 + max_systems * 1024;
+    // a dense system of n beads takes n^2 entries for its main lists and as
+    // many again when every bead is charged (whole columns per unit)
+    const int64_t list_cap = max_beads * 512 + max_systems * 4096;
     list_alloc_.reset(list_cap);
     lists_.alloc(list_cap);
+    bead_order_.alloc(max_beads);
     OCM_CK(cudaMallocHost(&h_overflow_, sizeof(int) * max_systems));
     std::memset(h_overflow_, 0, sizeof(int) * max_systems);
     OCM_CK(cudaMallocHost(&h_status_, sizeof(int) * max_systems));
@@ -1378,11 +1774,8 @@ BatchEngine::~BatchEngine() {
     if (copy_stream_) cudaStreamDestroy(copy_stream_);
 }
 
-// Shared memory of the per-system state: kBeadBytes per bead
-// (kBeadBytesGeneral with the general pair terms) and kFixedBytes.
-size_t BatchEngine::smem_bytes(int nmax, bool general) const {
-    return (size_t)nmax * (general ? kBeadBytesGeneral : kBeadBytes) + kFixedBytes;
-}
+// Shared memory of the per-system state of a class.
+size_t BatchEngine::smem_bytes(int nmax, int cls) const { return (size_t)nmax * kBeadBytes[cls] + kFixedBytes; }
 
 int64_t BatchEngine::footprint(const SystemDesc& d) {
     CompiledSystem c = compile_system(d);
@@ -1428,8 +1821,16 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
     if (slot < 0) throw Error(3, "[error] no free slot in the batch");
     const BondedPlan P = plan_bonded(c);
     const BlobLayout L = blob_layout(c, P);
-    const int npad = (int)align_up(n, 32);
-    const int maxn = initial_list_capacity(c, pos);
+    const PairPlan pairs = plan_pairs(c);
+    const int64_t nq = (int64_t)pairs.charged.size();
+    BatchSys R{};
+    R.cls = pairs.cls;
+    R.n = (int)n;
+    R.nq = (int)nq;
+    R.maxn = initial_list_capacity(n, nullptr, pair_split((int)n, kSplitUnits), pairs.main_rc, pos);
+    R.maxq = nq ? initial_list_capacity(nq, pairs.charged.data(), pair_split((int)nq, kSplitCharged), pairs.dh_rc, pos) : 0;
+    R.main_rc = (float)pairs.main_rc;
+    R.dh_rc = (float)pairs.dh_rc;
     const int64_t boff = beads_.alloc(n, 1);
     if (boff < 0) throw Error(3, "[error] batch bead capacity exhausted");
     const int64_t blob_off = blob_.alloc(L.size, 256);
@@ -1437,7 +1838,7 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
         beads_.release(boff, n);
         throw Error(3, "[error] batch parameter memory exhausted");
     }
-    const int64_t list_size = (int64_t)maxn * npad;
+    const int64_t list_size = list_entries(R);
     const int64_t list_off = list_alloc_.alloc(list_size, 64);
     if (list_off < 0) {
         beads_.release(boff, n);
@@ -1507,11 +1908,10 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
         put(L.off_ex_start, c.ex_start.data(), 4 * c.ex_start.size());
         put(L.off_ex, ex.data(), 4 * ex.size());
     }
+    put(L.off_qidx, pairs.charged.data(), 2 * pairs.charged.size());
 
-    BatchSys R{};
     R.bead_off = boff;
     R.blob_off = blob_off;
-    R.n = (int)n;
     R.nt = (int)((n + 31) / 32);
     R.n_bonds = (int)P.bonds.size();
     R.n_angles = (int)P.angles.size();
@@ -1521,9 +1921,8 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
     R.rb_p = L.rb_p; R.rb_ij = L.rb_ij; R.ra_ij = L.ra_ij; R.ra_k = L.ra_k; R.rd = L.rd; R.rgd = L.rgd;
     R.rfla = L.rfla; R.rfld = L.rfld;
     R.rcb = L.rcb; R.rca = L.rca; R.rcd = L.rcd; R.rgs = L.rgs; R.rgl = L.rgl;
-    R.off_ex_start = L.off_ex_start; R.off_ex = L.off_ex;
+    R.off_ex_start = L.off_ex_start; R.off_ex = L.off_ex; R.off_qidx = L.off_qidx;
     R.skin = kBatchSkin;
-    R.maxn = maxn;
     R.list_off = list_off;
     R.active = 1;
     R.pc = c.pc;
@@ -1545,7 +1944,10 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
         py[i] = pos[3 * i + 1];
         pz[i] = pos[3 * i + 2];
     }
+    std::vector<uint16_t> iota(n);  // bead order of the pair passes until the first launch sorts it
+    std::iota(iota.begin(), iota.end(), (uint16_t)0);
     cudaStream_t s = copy_stream_;
+    OCM_CK(cudaMemcpyAsync(bead_order_.p + boff, iota.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
     OCM_CK(cudaMemcpyAsync(blob_dev_.p + blob_off, blob.data(), L.size, cudaMemcpyHostToDevice, s));
     OCM_CK(cudaMemcpyAsync(x_.p + boff, px.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
     OCM_CK(cudaMemcpyAsync(y_.p + boff, py.data(), n * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -1582,9 +1984,7 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
     S.steps_done = (uint64_t)steps_done;
     S.list_off = list_off;
     S.list_size = list_size;
-    S.maxn = maxn;
-    S.terms = c.pc.terms;
-    S.labels = c.pc.uses_labels != 0;
+    S.cls = R.cls;
     for (int k = 0; k < kNumSlots; ++k) S.slot_group[k] = c.slot_group[k];
     const double nt = (double)R.nt;
     S.cost = nt * (nt + 1) / 2 + 0.05 * (double)n;
@@ -1592,18 +1992,15 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
     return slot;
 }
 
-void BatchEngine::launch(bool integrate, bool energy, int k, const std::vector<int32_t>& order,
-                         cudaStream_t s, const std::vector<int32_t>* order_k) {
-    bool general = false;
-    int terms = 0;
+void BatchEngine::launch(bool integrate, int k, const std::vector<int32_t>& order, cudaStream_t s,
+                         const std::vector<int32_t>* order_k, uint32_t slots_enabled) {
+    int cls = kClassGo;
     size_t bonded_max = 0;
     for (int32_t q : order) {
-        terms |= slots_[q].terms;
-        general = general || slots_[q].labels;
+        cls = std::max(cls, slots_[q].cls);
         bonded_max = std::max(bonded_max, (size_t)sys_host_[q].bonded_bytes);
     }
-    if (terms & ~(kTermEXV | kTermDH)) general = true;
-    const size_t smem = smem_bytes(nmax_, general);
+    const size_t smem = smem_bytes(nmax_, cls);
     const size_t want = list_smem_kib_ >= 0 ? smem + bonded_max + (size_t)list_smem_kib_ * 1024 : 0;
     int optin = 0;
     OCM_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
@@ -1630,15 +2027,11 @@ void BatchEngine::launch(bool integrate, bool energy, int k, const std::vector<i
     a.energy = energy_.p;
     a.forces = forces_.p;
     a.lists = lists_.p;
-    a.slots_enabled = 0xffffffffu;
+    a.bead_order = bead_order_.p;
+    a.slots_enabled = slots_enabled;
     a.split_beads = integrate ? split_beads_ : 0;
-    a.split_bead_bytes = general ? kBeadBytesGeneral : kBeadBytes;
-    const int grid = (int)order.size();
-    if (general)
-        launch_batch_threads<15, true>(threads_, a, grid, smem, s, integrate, energy, num_sms_, want);
-    else
-        launch_batch_threads<kTermEXV | kTermDH, false>(threads_, a, grid, smem, s, integrate, energy, num_sms_,
-                                                         want);
+    a.split_bead_bytes = kBeadBytes[cls];
+    launch_batch(cls, threads_, a, (int)order.size(), smem, s, integrate, num_sms_, want);
 }
 
 void BatchEngine::run(int32_t k, bool sync) {
@@ -1663,7 +2056,7 @@ void BatchEngine::run(int32_t k, bool sync) {
     }
     OCM_CK(cudaStreamWaitEvent(stream_, ev_copy_, 0));
     OCM_CK(cudaEventRecord(ev0_, stream_));
-    if (!order.empty()) launch(true, false, k, order, stream_, balanced_ ? &ks : nullptr);
+    if (!order.empty()) launch(true, k, order, stream_, balanced_ ? &ks : nullptr, 0xffffffffu);
     OCM_CK(cudaEventRecord(ev1_, stream_));
     OCM_CK(cudaMemcpy2DAsync(h_overflow_, sizeof(int), &sys_.p[0].overflow, sizeof(BatchSys),
                              sizeof(int), max_systems_, cudaMemcpyDeviceToHost, stream_));
@@ -1765,9 +2158,11 @@ void BatchEngine::grow_lists() {
         if (!h_overflow_[s] || !slots_[s].used) continue;
         h_overflow_[s] = 0;
         Slot& S = slots_[s];
-        const int npad = (int)align_up(S.n, 32);
-        const int maxn = (int)std::min<int64_t>(std::max<int64_t>(1, S.n - 1), align_up(S.maxn * 3 / 2 + 8, 4));
-        const int64_t size = (int64_t)maxn * npad;
+        BatchSys R = sys_host_[s];
+        auto grown = [](int cap, int limit) { return std::min((int)align_up(cap * 3 / 2 + 8, 4), limit); };
+        R.maxn = grown(R.maxn, unit_capacity_limit(R.n, pair_split(R.n, kSplitUnits)));
+        if (R.nq) R.maxq = grown(R.maxq, unit_capacity_limit(R.nq, pair_split(R.nq, kSplitCharged)));
+        const int64_t size = list_entries(R);
         list_alloc_.release(S.list_off, S.list_size);
         const int64_t off = list_alloc_.alloc(size, 64);
         if (off < 0) {
@@ -1777,14 +2172,13 @@ void BatchEngine::grow_lists() {
         }
         S.list_off = off;
         S.list_size = size;
-        S.maxn = maxn;
-        sys_host_[s].list_off = off;
-        sys_host_[s].maxn = maxn;
-        sys_host_[s].overflow = 0;
+        R.list_off = off;
+        R.overflow = 0;
+        sys_host_[s] = R;
         BatchSys* dst = sys_.p + s;
         OCM_CK(cudaMemcpyAsync(&dst->list_off, &sys_host_[s].list_off, sizeof(long long),
                                cudaMemcpyHostToDevice, stream_));
-        OCM_CK(cudaMemcpyAsync(&dst->maxn, &sys_host_[s].maxn, sizeof(int), cudaMemcpyHostToDevice, stream_));
+        OCM_CK(cudaMemcpyAsync(&dst->maxn, &sys_host_[s].maxn, 2 * sizeof(int), cudaMemcpyHostToDevice, stream_));
         OCM_CK(cudaMemcpyAsync(&dst->overflow, &sys_host_[s].overflow, sizeof(int),
                                cudaMemcpyHostToDevice, stream_));
         OCM_CK(cudaStreamSynchronize(stream_));
@@ -1851,25 +2245,7 @@ void BatchEngine::get_state(int64_t slot, uint32_t groups, double* forces, doubl
     std::vector<int32_t> order{(int32_t)slot};
     OCM_CK(cudaStreamWaitEvent(stream_, ev_copy_, 0));
     OCM_CK(cudaMemsetAsync(energy_.p + slot * kNumSlots, 0, kNumSlots * sizeof(double), stream_));
-    // The eval kernel reads slots_enabled from the args.
-    {
-        bool general = S.labels || (S.terms & ~(kTermEXV | kTermDH));
-        const size_t smem = smem_bytes(nmax_, general);
-        OCM_CK(cudaMemcpyAsync(order_.p, order.data(), sizeof(int32_t), cudaMemcpyHostToDevice, stream_));
-        OCM_CK(cudaMemsetAsync(head_.p, 0, sizeof(int32_t), stream_));
-        BatchArgs a{};
-        a.sys = sys_.p; a.order = order_.p; a.n_order = 1; a.head = head_.p;
-        a.x = x_.p; a.y = y_.p; a.z = z_.p; a.vx = vx_.p; a.vy = vy_.p; a.vz = vz_.p;
-        a.blob = blob_dev_.p; a.k = 0; a.nmax = nmax_; a.energy = energy_.p; a.forces = forces_.p;
-        a.lists = lists_.p;
-        a.slots_enabled = en;
-        const size_t want = list_smem_kib_ >= 0
-                                ? smem + (size_t)sys_host_[slot].bonded_bytes + (size_t)list_smem_kib_ * 1024
-                                : 0;
-        if (general) launch_batch_threads<15, true>(threads_, a, 1, smem, stream_, false, true, num_sms_, want);
-        else launch_batch_threads<kTermEXV | kTermDH, false>(threads_, a, 1, smem, stream_, false, true, num_sms_,
-                                                              want);
-    }
+    launch(false, 0, order, stream_, nullptr, en);
     std::vector<float> f(3 * nmax_);
     double e[kNumSlots];
     int bad = 0;
@@ -1913,7 +2289,7 @@ void BatchEngine::slot_stats(int64_t slot, int32_t* builds, int32_t* capacity) {
     int b = 0;
     OCM_CK(cudaMemcpy(&b, &sys_.p[slot].builds, sizeof(int), cudaMemcpyDeviceToHost));
     *builds = b;
-    *capacity = slots_[slot].maxn;
+    *capacity = sys_host_[slot].maxn;
 }
 
 // Scatter / gather of many slots' states through one pinned staging buffer

@@ -36,7 +36,10 @@ struct BatchSys {
     int rb_p, rb_ij, ra_ij, ra_k, rd, rgd, rfla, rfld;
     int rcb, rca, rcd, rgs, rgl;
     int off_ex_start, off_ex;                // exclusion CSR (j | bits << 24)
-    int maxn;              // neighbour-list entries per bead
+    int off_qidx;          // charged beads (u16, increasing)
+    int cls, nq;           // class of the pair terms, charged beads with a list of their own
+    float main_rc, dh_rc;  // cutoffs of the main and the charged lists (0: no such pairs)
+    int maxn, maxq;        // entries per unit of the main and of the charged lists
     int active;
     int overflow;          // set by the kernel when a list did not fit
     int builds;            // list builds in the last chunk
@@ -115,22 +118,22 @@ class BatchEngine {
         int64_t blob_off = 0, blob_size = 0;
         uint64_t steps_target = 0, steps_done = 0;
         double cost = 0;
-        int terms = 0;
-        bool labels = false;
+        int cls = 0;
         int slot_group[kNumSlots];
         int64_t list_off = 0, list_size = 0;
-        int maxn = 0;
         bool failed = false;  // blew up: no longer advanced
     };
     void grow_lists();
     void sync_steps();
-    void launch(bool integrate, bool energy, int k, const std::vector<int32_t>& order,
-                cudaStream_t s, const std::vector<int32_t>* order_k = nullptr);
+    // One launch over the slots in `order`: k MD steps (or order_k of them
+    // each), or one evaluation of the enabled terms.
+    void launch(bool integrate, int k, const std::vector<int32_t>& order, cudaStream_t s,
+                const std::vector<int32_t>* order_k, uint32_t slots_enabled);
     // Estimated time of one MD step of an n-bead system (arbitrary units):
     // the kernel's per-step time grows with n, with a floor set by the
     // per-step barriers of small systems.
     static double step_cost(int64_t n) { return (double)std::max<int64_t>(n, 150); }
-    size_t smem_bytes(int nmax, bool general) const;
+    size_t smem_bytes(int nmax, int cls) const;
 
     int device_;
     int64_t max_systems_, max_beads_;
@@ -146,7 +149,7 @@ class BatchEngine {
     DevBuf<double> x_, y_, z_;
     DevBuf<float> vx_, vy_, vz_;
     DevBuf<unsigned char> blob_dev_;
-    DevBuf<uint16_t> lists_;
+    DevBuf<uint16_t> lists_, bead_order_;
     int* h_overflow_ = nullptr;  // pinned copy of the records' overflow flags
     int* h_status_ = nullptr;    // pinned copy of the records' status words
     int* h_check_ = nullptr;     // pinned: non-finite values found by the upload check

@@ -1,0 +1,107 @@
+"""The batched kernel's classes of systems (excluded volume + Debye-Hueckel;
+Lennard-Jones + Debye-Hueckel with a longer Debye-Hueckel cutoff; everything
+else): forces and energies against the FP64 oracle, and trajectories that do
+not depend on which classes a launch holds nor on list overflow."""
+import numpy as np
+import pytest
+
+from conftest import rel_force_err
+
+pytestmark = pytest.mark.gpu
+
+FORCE_TOL = 1e-4   # FP32 pair arithmetic, the bar of the parity tests
+ENERGY_TOL = 1e-5
+
+
+def _chain(kind, n, seed):
+    """A coil of n beads: "go" is the Go protein; "hps" swaps the excluded
+    volume for both Lennard-Jones terms and lets Debye-Hueckel reach 3.5 nm;
+    "general" gives one bead another attractive sigma; "dh" keeps
+    Debye-Hueckel alone; "neutral" has no charge at all."""
+    from opencafemol_gb300 import synth
+    s = synth.go_protein(n, seed)
+    if kind in ("hps", "general"):
+        rng = np.random.default_rng(seed)
+        sig = rng.uniform(0.35, 0.45, n)
+        ratio = 2.0 / np.sort(sig)[-2:].mean()
+        s.exv = None
+        s.ljr = synth.PairTerm(ratio=ratio, p0=np.full(n, 0.8), p1=sig, ign_bond=3)
+        s.lja = synth.PairTerm(ratio=ratio, p0=rng.uniform(0.0, 0.8, n), p1=sig.copy(), ign_bond=3)
+        s.dh.ratio = 3.5 / synth.debye_length(300.0, 0.15)
+        if kind == "general":
+            s.lja.p1[n // 2] = s.ljr.p1[n // 2] * 0.99
+    elif kind == "dh":
+        s.exv = None
+    elif kind == "neutral":
+        s.dh = None
+    return s
+
+
+def _check_state(batch, slot, system, spec):
+    from oracle import oracle
+    f, e = batch.state(slot)
+    f_ref, e_ref = oracle.evaluate(spec)
+    assert rel_force_err(f, f_ref) <= FORCE_TOL
+    for g, name in enumerate(system.group_names()):
+        assert abs(e[g] - e_ref[name]) <= ENERGY_TOL * max(1.0, abs(e_ref[name])), name
+
+
+@pytest.mark.parametrize("kind", ["go", "hps", "general", "dh", "neutral"])
+@pytest.mark.parametrize("n", [5, 33, 64, 129, 257, 513, 800])
+def test_class_forces_and_group_masks(gpu, kind, n):
+    """Sizes around the edges of the pair split and of a cluster."""
+    from opencafemol_gb300 import synth
+    spec = _chain(kind, n, 40 + n)
+    system = synth.build_system(spec)
+    b = gpu.Batch(max_systems=1, max_total_beads=1024, max_beads_per_system=1024)
+    slot = b.admit(system, spec.pos, seed=1, n_steps=1)
+    _check_state(b, slot, system, spec)
+    total, masked = b.state(slot)[0], np.zeros((n, 3))
+    for g in range(len(system.group_names())):
+        masked += b.state(slot, groups=1 << g)[0]
+    assert np.allclose(masked, total, rtol=0, atol=1e-5 * max(1.0, np.abs(total).max()))
+
+
+def test_same_alone_and_among_other_classes(gpu):
+    """The kernel is chosen by the classes of the whole launch, the inner
+    loops by each system's own class: a system's bits are the same alone and
+    with any other class, in any launch shape, for any chunking."""
+    from opencafemol_gb300 import synth
+    kinds = [("go", 70), ("hps", 150), ("general", 90), ("hps", 400), ("go", 300), ("neutral", 40)]
+    specs = [_chain(k, n, 60 + n) for k, n in kinds]
+    systems = [synth.build_system(s) for s in specs]
+    def run(which, threads, chunks):
+        b = gpu.Batch(max_systems=len(which), max_total_beads=2048, max_beads_per_system=512)
+        b.set_threads(threads)
+        slots = [b.admit(systems[k], specs[k].pos, seed=5 + k, n_steps=120) for k in which]
+        for c in chunks:
+            b.run(c)
+        return {k: (b.positions(s), b.velocities(s)) for k, s in zip(which, slots)}
+    mix = run(range(len(kinds)), 512, [120])
+    again = run([0, 1, 3, 4], 256, [7, 50, 63])  # without the general class
+    for k in range(len(kinds)):
+        alone = run([k], 512, [60, 60])[k]
+        for other in (mix[k],) + ((again[k],) if k in again else ()):
+            assert np.array_equal(alone[0], other[0]) and np.array_equal(alone[1], other[1]), kinds[k]
+
+
+@pytest.mark.parametrize("kind", ["go", "hps", "general"])
+@pytest.mark.parametrize("n", [60, 200, 600])
+def test_overflow_scan_is_bit_identical(gpu, kind, n):
+    """Lists sized from a straight chain overflow on the coil's positions:
+    that launch scans, with the bits of a run whose lists were large enough."""
+    from opencafemol_gb300 import synth
+    spec = _chain(kind, n, 80 + n)
+    system = synth.build_system(spec)
+    straight = np.zeros((n, 3))
+    straight[:, 0] = 0.38 * np.arange(n)
+    v0 = np.random.default_rng(2).normal(scale=0.2, size=(n, 3)).astype(np.float32).astype(np.float64)
+    out = []
+    for start in (straight, spec.pos):
+        b = gpu.Batch(max_systems=1, max_total_beads=1024, max_beads_per_system=1024)
+        slot = b.admit(system, start, temperature=300.0, seed=9, n_steps=60)
+        b.set_positions_many([slot], spec.pos, v0)
+        b.run(30)
+        b.run(30)
+        out.append((b.positions(slot), b.velocities(slot)))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])

@@ -35,6 +35,8 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall",
              "-I", str(CUDA_HOME / "include"), "-I", str(INCLUDE)]
 
 CU_SOURCES = ["plain_engine.cu", "batch_engine.cu"]
+# per-unit flags: the batched kernels' fused multiply-adds are explicit
+CU_FLAGS = {"batch_engine.cu": ["--fmad=false"]}
 CXX_SOURCES = ["host_system.cpp", "tables.cpp", "capi.cpp", "minimize.cpp"]
 
 
@@ -72,7 +74,7 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> Path:
         objs.append(obj)
         if _stale(obj, src, deps) or ptxas_info:
             extra = ["-Xptxas", "-v"] if ptxas_info else []
-            jobs.append(([NVCC, *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(obj)], name))
+            jobs.append(([NVCC, *NVCC_FLAGS, *CU_FLAGS.get(name, []), *extra, "-c", str(src), "-o", str(obj)], name))
     for name in CXX_SOURCES:
         src, obj = CSRC / name, OBJ / (name + ".o")
         objs.append(obj)

@@ -20,7 +20,10 @@
 //             and blow-up checks.
 // No atomics on forces: every bead's force is a sum in a fixed order, so a
 // system gives the same trajectory alone, in any mix, for any chunking and
-// for any threads per CTA.
+// for any threads per CTA.  The unit is compiled with contraction off and
+// its fused multiply-adds are written out: the kernels inline the same code
+// many times over, and a product contracted into a sum in one copy and not
+// in another would let a system's bits depend on the launch shape.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,13 +47,12 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxClusters = 64;  // 2048 beads per system
 // Pair work of a bead is split over S adjacent lanes (S = 1, 2, 4 or 8, the
-// largest with n * S <= kSplitUnits); sub-lane s sums the partners whose j
+// largest with n * S <= split_units of the class); sub-lane s sums the partners whose j
 // lies in [s*n/S, (s+1)*n/S).  S depends on n alone, so the FP32 sums, and
 // the results, do not depend on the threads per CTA (a CTA with fewer
 // threads walks the units in more passes).  The charged beads' partners are
-// split the same way among the nq charged beads (kSplitCharged).
-constexpr int kSplitUnits = 512;
-constexpr int kSplitCharged = 128;
+// split the same way among the nq charged beads (charged_units).
+constexpr int kSplitMost = 512;
 constexpr int kMaxSplit = 8;
 // Beads are ordered by their longest sub-list (bucket sort over this many
 // buckets), so the 32 lanes of a pair pass carry work of similar length.
@@ -74,7 +76,7 @@ constexpr int kSortBuilds = 4;
 // disordered chains of 50..400 beads, 3.5 nm against 2.0 nm: one combined
 // list holds about 2.5 times as many entries).  General keeps one list whose
 // entries carry the excluded terms.
-// Issue-bound: an excluded-volume entry takes about 23 instructions and one
+// Issue-bound: an excluded-volume entry takes about 21 instructions and one
 // 16-byte gather where the combined walk took over 40 and two.  Per 100 steps
 // with the read-out, against one combined list for all: 512 Go proteins of
 // 50..800 beads 2.92 -> 2.30 ms, 300 disordered chains 6.74 -> 1.95 ms, 24
@@ -91,7 +93,7 @@ constexpr int kClassGeneral = 2;
 // buckets, alignment).
 constexpr int kBeadBytes[3] = {104, 112, 120};
 constexpr size_t kFixedBytes =
-    (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kSplitUnits + 2 * kSplitCharged + 4 * kSortBuckets + 16;
+    (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kSplitMost + kSplitMost / 2 + 4 * kSortBuckets + 16;
 // A force component beyond this (kJ/mol/nm) marks a blown-up system: far
 // above any physical coarse-grained force, and the bound of the plain
 // engine's fixed-point accumulators.
@@ -102,6 +104,13 @@ __host__ __device__ __forceinline__ int pair_split(int n, int units) {
     while (S < kMaxSplit && n * S * 2 <= units) S <<= 1;
     return S;
 }
+// Units a small system is split into.  Every pass costs about 150 instructions
+// beside its entries, so the short excluded-volume entries want fewer units
+// (against 512: 24 small proteins 549 -> 523 us, 1400 peptides 2.26 -> 2.04
+// ms per 100 steps), the longer Lennard-Jones ones more (256 against 512:
+// 300 disordered chains 1.85 against 1.76 ms).
+__host__ __device__ __forceinline__ int split_units(int cls) { return cls == 0 ? 256 : kSplitMost; }
+__host__ __device__ __forceinline__ int charged_units(int cls) { return split_units(cls) / 4; }
 
 struct BatchArgs {
     BatchSys* sys;
@@ -166,10 +175,6 @@ __device__ __forceinline__ float3 neg3(float3 a) { return make_float3(-a.x, -a.y
 __device__ __forceinline__ float3 shfl_up3(float3 v, int d) {
     return make_float3(__shfl_up_sync(kFull, v.x, d), __shfl_up_sync(kFull, v.y, d), __shfl_up_sync(kFull, v.z, d));
 }
-__device__ __forceinline__ float3 shfl3(float3 v, int src) {
-    return make_float3(__shfl_sync(kFull, v.x, src), __shfl_sync(kFull, v.y, src), __shfl_sync(kFull, v.z, src));
-}
-
 // Per-term energy accumulators: FP64 sums of the FP32 per-term energies.
 struct EnergyAcc {
     double e[kNumSlots];
@@ -198,20 +203,24 @@ struct Bonded {
     const uint32_t* gl;     // type << 30 | role << 28 | term index
 };
 
-// Bond b: force on its first bead (the second gets the negation), energy.
-__device__ __forceinline__ float3 bond_force(const Bonded& B, int b, const float4* sx, const float* sxl, int ns,
-                                             float& en, int& slot) {
-    const uint32_t ij = B.bij[b];
-    const int kind = (int)(ij >> 30);
+// Bond b from the float-float separation of its beads: force on the first
+// bead (the second gets the negation), energy.
+__device__ __forceinline__ float3 bond_force(const Bonded& B, int b, float3 dh, float3 dl, float& en, int& slot) {
+    const int kind = (int)(B.bij[b] >> 30);
     slot = bond_slot(kind);
-    const int bi = ij & 0xFFFF, bj = (ij >> 16) & 0x3FFF;
     const float4 bp = B.bpar[b];
-    float3 dh, dl;
-    ff_sep(sx[bi], lo3(sxl, ns, bi), sx[bj], lo3(sxl, ns, bj), dh, dl);
     const float3 d = make_float3(dh.x + dl.x, dh.y + dl.y, dh.z + dl.z);
     const float delta = ff_bond_delta(dh, dl, bp.z, bp.w);
     const float sc = bond_scalar(kind, norm2(d), delta, bp.x, bp.y, bp.z, en);
     return make_float3(-sc * d.x, -sc * d.y, -sc * d.z);
+}
+__device__ __forceinline__ float3 bond_force(const Bonded& B, int b, const float4* sx, const float* sxl, int ns,
+                                             float& en, int& slot) {
+    const uint32_t ij = B.bij[b];
+    const int bi = ij & 0xFFFF, bj = (ij >> 16) & 0x3FFF;
+    float3 dh, dl;
+    ff_sep(sx[bi], lo3(sxl, ns, bi), sx[bj], lo3(sxl, ns, bj), dh, dl);
+    return bond_force(B, b, dh, dl, en, slot);
 }
 
 // Angle a: forces on its first (f1) and last (f3) bead; the middle one
@@ -225,34 +234,41 @@ __device__ __forceinline__ void angle_force(const Bonded& B, int a, const float4
     fla_forces(u, v, B.ak[a], B.fla[g.y >> 16], f1, f3, en);
 }
 
-// Dihedral q: forces on its four beads, energy and slot.
-__device__ __forceinline__ void dihedral_force(const Bonded& B, int q, const float4* sx, const float* sxl, int ns,
+// Dihedral q of geometry g: forces on its four beads, energy and slot.
+__device__ __forceinline__ void dihedral_force(const Bonded& B, int q, const Torsion& g, float3 F, float3 G, float3 H,
                                                float3& f1, float3& f2, float3& f3, float3& f4, float& en,
                                                int& slot) {
     const uint4 qd = B.drec[q];
     const bool gauss = (qd.x >> 31) != 0;
     slot = gauss ? kSlotGD : kSlotFLD;
+    if (gauss) {
+        const float2 gp = B.gdp[qd.z];
+        gauss_dihedral_forces(g, F, G, H, __uint_as_float(qd.w), gp.x, gp.y, f1, f2, f3, f4, en);
+    } else {
+        fld_forces(g, F, G, H, __uint_as_float(qd.w), B.fld[qd.z], f1, f2, f3, f4, en);
+    }
+}
+__device__ __forceinline__ void dihedral_force(const Bonded& B, int q, const float4* sx, const float* sxl, int ns,
+                                               float3& f1, float3& f2, float3& f3, float3& f4, float& en,
+                                               int& slot) {
+    const uint4 qd = B.drec[q];
     const int qi = qd.x & 0xFFFF, qj = (qd.x >> 16) & 0x7FFF, qk = qd.y & 0xFFFF, ql = qd.y >> 16;
     const float3 F = ffsep(sx, sxl, ns, qj, qi);
     const float3 G = ffsep(sx, sxl, ns, qk, qj);
     const float3 H = ffsep(sx, sxl, ns, qk, ql);
-    if (gauss) {
-        const float2 gp = B.gdp[qd.z];
-        gauss_dihedral_forces(F, G, H, __uint_as_float(qd.w), gp.x, gp.y, f1, f2, f3, f4, en);
-    } else {
-        fld_forces(F, G, H, __uint_as_float(qd.w), B.fld[qd.z], f1, f2, f3, f4, en);
-    }
+    dihedral_force(B, q, torsion_geometry(F, G, H), F, G, H, f1, f2, f3, f4, en, slot);
 }
 
 __device__ __forceinline__ bool slot_on(uint32_t slots_en, int slot) { return (slots_en >> slot) & 1u; }
 
 // Bonded force on bead b = I * 32 + lane of cluster I (one warp).  The lane
-// evaluates every chain-local term starting at b (bonds from b to b+1, b+2
-// or b+3, angles b..b+2, dihedrals b..b+3) once, keeping its contributions to b..b+3; the
-// lanes then add what lanes 1..3 below them send up, in a fixed order, and
-// the three contributions that cross into cluster I + 1 go to carry[I].
-// Terms that are not chain-local are evaluated by each of their beads
-// (gather entries) and only that bead's share is kept.
+// evaluates every chain-local term starting at b (bonds from b to b+1, b+2 or b+3, angles b..b+2, dihedrals
+// b..b+3) once, keeping its contributions to b..b+3; the lanes then add what
+// lanes 1..3 below them send up, in a fixed order, and the three
+// contributions that cross into cluster I + 1 go to carry[I].  Terms that
+// are not chain-local are evaluated by each of their beads (gather entries)
+// and only that bead's share is kept.  The three chain bonds that start at
+// b, b+1 and b+2 and their cross products serve all of the lane's terms.
 template <bool ENERGY>
 __device__ __forceinline__ float3 bonded_cluster(const Bonded& B, int I, int n, int lane, const float4* sx,
                                                  const float* sxl, int ns, uint32_t slots_en, float3* carry,
@@ -260,39 +276,67 @@ __device__ __forceinline__ float3 bonded_cluster(const Bonded& B, int I, int n, 
     const int b = I * 32 + lane;
     float3 o0 = make_float3(0.f, 0.f, 0.f), o1 = o0, o2 = o0, o3 = o0;
     if (b < n) {
+        const int b1 = min(b + 1, n - 1), b2 = min(b + 2, n - 1);
+        const float4 x1 = sx[b1];
+        const float3 l1 = lo3(sxl, ns, b1);
+        float3 h01, e01;
+        ff_sep(sx[b], lo3(sxl, ns, b), x1, l1, h01, e01);
         for (int t = B.cb[b]; t < B.cb[b + 1]; ++t) {
             float en;
             int sl;
-            const float3 f = bond_force(B, t, sx, sxl, ns, en, sl);
+            const int d = (int)((B.bij[t] >> 16) & 0x3FFF) - b;
+            float3 dh = h01, dl = e01;
+            if (d > 1) ff_sep(sx[b], lo3(sxl, ns, b), sx[b + d], lo3(sxl, ns, b + d), dh, dl);
+            const float3 f = bond_force(B, t, dh, dl, en, sl);
             if (!slot_on(slots_en, sl)) continue;
             add3(o0, f);
-            const int d = (int)((B.bij[t] >> 16) & 0x3FFF) - b;
             if (d == 1) add3(o1, neg3(f));
             else if (d == 2) add3(o2, neg3(f));
             else add3(o3, neg3(f));
             if (ENERGY) ea.e[sl] += (double)en;
         }
+        const float4 x2 = sx[b2];
+        const float3 l2 = lo3(sxl, ns, b2);
+        float3 dh, dl;
+        ff_sep(x1, l1, x2, l2, dh, dl);
+        const float3 d01 = make_float3(h01.x + e01.x, h01.y + e01.y, h01.z + e01.z);
+        const float3 d12 = make_float3(dh.x + dl.x, dh.y + dl.y, dh.z + dl.z);
+        const float3 A = cross3(d01, d12);
+        const float AA = fmaxf(norm2(A), 1e-30f);
         if (slot_on(slots_en, kSlotFLA))
             for (int t = B.ca[b]; t < B.ca[b + 1]; ++t) {
-                float3 f1, f3;
+                // with u = -d01, v = d12 and n = u x v = -A:
+                // f1 = -dE/(|u|^2 |n|) u x n, f3 = dE/(|v|^2 |n|) v x n
                 float en;
-                angle_force(B, t, sx, sxl, ns, f1, f3, en);
+                const float nlen = sqrtf(AA);
+                const float theta = atan2f(nlen, -dot3(d01, d12));
+                const float dE = fla_slope(theta, B.ak[t], B.fla[B.aij[t].y >> 16], en);
+                const float3 un = cross3(d01, A), vn = cross3(d12, A);
+                const float c1 = -dE / (norm2(d01) * nlen), c3 = -dE / (norm2(d12) * nlen);
+                const float3 f1 = make_float3(c1 * un.x, c1 * un.y, c1 * un.z);
+                const float3 f3 = make_float3(c3 * vn.x, c3 * vn.y, c3 * vn.z);
                 add3(o0, f1);
                 add3(o2, f3);
                 add3(o1, make_float3(-f1.x - f3.x, -f1.y - f3.y, -f1.z - f3.z));
                 if (ENERGY) ea.e[kSlotFLA] += (double)en;
             }
-        for (int t = B.cd[b]; t < B.cd[b + 1]; ++t) {
-            float3 f1, f2, f3, f4;
-            float en;
-            int sl;
-            dihedral_force(B, t, sx, sxl, ns, f1, f2, f3, f4, en, sl);
-            if (!slot_on(slots_en, sl)) continue;
-            add3(o0, f1);
-            add3(o1, f2);
-            add3(o2, f3);
-            add3(o3, f4);
-            if (ENERGY) ea.e[sl] += (double)en;
+        if (B.cd[b] < B.cd[b + 1]) {
+            ff_sep(x2, l2, sx[b + 3], lo3(sxl, ns, b + 3), dh, dl);
+            const float3 H = make_float3(dh.x + dl.x, dh.y + dl.y, dh.z + dl.z);
+            const float3 F = neg3(d01), G = neg3(d12);
+            const Torsion g = torsion_geometry(F, G, H, A, AA);
+            for (int t = B.cd[b]; t < B.cd[b + 1]; ++t) {
+                float3 f1, f2, f3, f4;
+                float en;
+                int sl;
+                dihedral_force(B, t, g, F, G, H, f1, f2, f3, f4, en, sl);
+                if (!slot_on(slots_en, sl)) continue;
+                add3(o0, f1);
+                add3(o1, f2);
+                add3(o2, f3);
+                add3(o3, f4);
+                if (ENERGY) ea.e[sl] += (double)en;
+            }
         }
     }
     // contributions of the three chain positions below, in the order
@@ -302,19 +346,19 @@ __device__ __forceinline__ float3 bonded_cluster(const Bonded& B, int I, int n, 
     if (lane >= 1) add3(fb, u1);
     if (lane >= 2) add3(fb, u2);
     if (lane >= 3) add3(fb, u3);
-    // what lanes 29..31 send into the next cluster's first three beads
-    const float3 a1 = shfl3(o1, 31), a2 = shfl3(o2, 30), a3 = shfl3(o3, 29);
-    const float3 b2 = shfl3(o2, 31), b3 = shfl3(o3, 30);
-    const float3 c3 = shfl3(o3, 31);
-    if (lane == 0) {
-        float3 c0 = a1;
+    // what lanes 29..31 send into the next cluster's first three beads: lane
+    // 29 o3 to the first, lane 30 o2 and o3 to the first and second, lane 31
+    // o1, o2 and o3 to the first, second and third
+    const float3 a2 = shfl_up3(o2, 1), a3 = shfl_up3(o3, 2), b3 = shfl_up3(o3, 1);
+    if (lane == 31) {
+        float3 c0 = o1;
         add3(c0, a2);
         add3(c0, a3);
-        float3 c1 = b2;
+        float3 c1 = o2;
         add3(c1, b3);
         carry[3 * I] = c0;
         carry[3 * I + 1] = c1;
-        carry[3 * I + 2] = c3;
+        carry[3 * I + 2] = o3;
     }
     if (b < n) {
         for (int g = B.gs[b]; g < B.gs[b + 1]; ++g) {
@@ -433,6 +477,12 @@ __device__ __forceinline__ void list_walk(const UnitList& L, int col, int cnt, F
     for (int g = shared; g < groups; ++g) four(*reinterpret_cast<const uint2*>(q + (size_t)g * L.cols * 4));
 }
 
+// Go and Hps entries are byte offsets of the partner's position (16 j, at
+// most 32768): an address without a shift.
+__device__ __forceinline__ float4 position_at(const float4* sx, uint32_t e) {
+    return *reinterpret_cast<const float4*>(reinterpret_cast<const unsigned char*>(sx) + e);
+}
+
 __device__ __forceinline__ uint32_t entry_of(uint2 e, int u) {
     const uint32_t w = u < 2 ? e.x : e.y;
     return u & 1 ? w >> 16 : w & 0xFFFFu;
@@ -449,7 +499,7 @@ __device__ __forceinline__ bool box_far(float4 x, float4 c, float4 h, float cut2
 // Main list of every unit, one thread per unit (bead i, range s): the j != i
 // of the range whose FP32 r^2 (canonical form) is below cut2, in increasing
 // j, so the list and every FP32 sum over it are deterministic.  Go and Hps
-// keep j alone and leave out the pairs that their short-range term excludes;
+// keep 16 j alone and leave out the pairs that their short-range term excludes;
 // General keeps j | excluded-term bits << 11 and leaves out the pairs that
 // every present term excludes.  Per cluster the 32 distance tests set bits
 // of a mask without a branch and only the set bits go on, with the
@@ -493,7 +543,7 @@ __device__ __forceinline__ void build_main(int n, int lg, float cut2, const floa
                     if (ew & drop) m &= ~(1u << ((ew & 0xFFFFFF) - jb));
                     ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
                 }
-                for (; m; m &= m - 1) list_put(L, cnt++, col, (uint32_t)(jb + __ffs(m) - 1));
+                for (; m; m &= m - 1) list_put(L, cnt++, col, (uint32_t)(jb + __ffs(m) - 1) << 4);
             } else {
                 for (; m; m &= m - 1) {
                     const int j = jb + __ffs(m) - 1;
@@ -505,7 +555,7 @@ __device__ __forceinline__ void build_main(int n, int lg, float cut2, const floa
             }
         }
         // padding: the dummy bead, or the bead itself with every term excluded
-        ucnt[col] = (uint16_t)list_close(L, cnt, col, CLS == kClassGeneral ? (uint32_t)i | 15u << 11 : (uint32_t)npad,
+        ucnt[col] = (uint16_t)list_close(L, cnt, col, CLS == kClassGeneral ? (uint32_t)i | 15u << 11 : (uint32_t)npad << 4,
                                          overflow);
     }
 }
@@ -540,10 +590,10 @@ __device__ __forceinline__ void build_charged(int nq, int lg, float cut2, const 
                 if (j == i) continue;
                 while ((ew & 0xFFFFFF) < j) ew = ++ep < e1 ? ex[ep] : 0x00FFFFFF;
                 if ((ew & 0xFFFFFF) == j && (ew & kTermDH << 24)) continue;
-                list_put(L, cnt++, u, (uint32_t)j);
+                list_put(L, cnt++, u, (uint32_t)j << 4);
             }
         }
-        qcnt[u] = (uint16_t)list_close(L, cnt, u, (uint32_t)npad, overflow);
+        qcnt[u] = (uint16_t)list_close(L, cnt, u, (uint32_t)npad << 4, overflow);
     }
 }
 
@@ -588,7 +638,8 @@ __device__ __forceinline__ void sort_beads(int n, int lg, const uint16_t* ucnt, 
 // ---------------------------------------------------------------------------
 // Pair arithmetic of the Go and Hps classes.  Every operation is rounded by
 // itself, so the list walk, the scan and every kernel that holds a class
-// give the same bits.  A pair outside the cutoff contributes exactly zero.
+// give the same bits.  A pair outside the cutoff contributes exactly zero (the
+// last select; whatever the arithmetic before it made of its distance).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
@@ -608,7 +659,7 @@ __device__ __forceinline__ void exv_pair(float4 xi, float4 xj, const PairConsts&
     const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
     const float r2 = norm2(d);
     const bool in = r2 < pc.exv_rc2;
-    const float ri = rcp_approx(in ? r2 : 1.f);
+    const float ri = rcp_approx(r2);
     const float S = __fadd_rn(xi.w, xj.w);
     const float S2 = __fmul_rn(S, S);
     const float u = __fmul_rn(S2, ri);
@@ -633,19 +684,18 @@ __device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float
     const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
     const float r2 = norm2(d);
     const bool in = r2 < pc.lja_rc2;
-    const float r2c = in ? r2 : 1.f;
-    const float rinv = rsqrtf(r2c);
+    const float rinv = rsqrtf(r2);
     const float ri = __fmul_rn(rinv, rinv);
     const float sg = __fadd_rn(xi.w, xj.w);
     const float sig2 = __fmul_rn(sg, sg);
     const float s2 = __fmul_rn(sig2, ri);
     const float s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
     const float s12 = __fmul_rn(s6, s6);
-    const bool core = r2c <= __fmul_rn(sig2, kTwoPow1_3);
+    const bool core = r2 <= __fmul_rn(sig2, kTwoPow1_3);
     const float er = __fadd_rn(lei.x, lej.x), el = __fadd_rn(lei.y, lej.y);
     const float t = __fmul_rn(__fmul_rn(24.f, ri), __fmaf_rn(2.f, s12, -s6));
     float s = __fmul_rn(core ? er : el, t);
-    const float r = __fmul_rn(r2c, rinv);
+    const float r = __fmul_rn(r2, rinv);
     float sw = 1.f;
     if (r > pc.lja_rs) {
         // OpenMM switching function S = 1 - 10x^3 + 15x^4 - 6x^5.
@@ -673,10 +723,9 @@ __device__ __forceinline__ void dh_pair(float4 xi, float4 xj, float qk, float qj
     const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
     const float r2 = norm2(d);
     const bool in = r2 < pc.dh_rc2;
-    const float r2c = in ? r2 : 1.f;
-    const float rinv = rsqrtf(r2c);
+    const float rinv = rsqrtf(r2);
     const float ri = __fmul_rn(rinv, rinv);
-    const float ex = exp2f(__fmul_rn(-__fmul_rn(r2c, rinv), pc.dh_inv_lambda_log2e));
+    const float ex = exp2f(__fmul_rn(-__fmul_rn(r2, rinv), pc.dh_inv_lambda_log2e));
     const float qq = __fmul_rn(qk, qj);
     const float s = __fmul_rn(__fmul_rn(__fmul_rn(qq, ex), __fadd_rn(pc.dh_inv_lambda, rinv)), ri);
     sub_force(f, in ? s : 0.f, d);
@@ -694,9 +743,7 @@ __device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 p0i, f
     e.zero();
     float sc = pair_scalar<15, ENERGY>(in ? r2 : pc.list_rc2, p0i, p0j, p1i, p1j, bits, pc, e);
     sc = in ? sc : 0.f;
-    fa.x -= sc * d.x;
-    fa.y -= sc * d.y;
-    fa.z -= sc * d.z;
+    sub_force(fa, sc, d);
     if (ENERGY && in) {
         // every pair is met from both of its beads
         ea.e[kSlotEXV] += 0.5 * (double)e.exv;
@@ -727,7 +774,7 @@ __device__ __forceinline__ float3 main_list(int i, int col, int cnt, const UnitL
         list_walk(L, col, cnt, [&](uint2 e) {
             float4 xj[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) xj[u] = sx[entry_of(e, u)];
+            for (int u = 0; u < 4; ++u) xj[u] = position_at(sx, entry_of(e, u));
 #pragma unroll
             for (int u = 0; u < 4; ++u) exv_pair<ENERGY>(xi, xj[u], pc, f, ea);
         });
@@ -738,8 +785,8 @@ __device__ __forceinline__ float3 main_list(int i, int col, int cnt, const UnitL
             float2 lej[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                xj[u] = sx[entry_of(e, u)];
-                lej[u] = P.le[entry_of(e, u)];
+                xj[u] = position_at(sx, entry_of(e, u));
+                lej[u] = P.le[entry_of(e, u) >> 4];
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) hps_pair<ENERGY>(xi, xj[u], lei, lej[u], pc, f, ea);
@@ -774,8 +821,8 @@ __device__ __forceinline__ float3 charged_list(int i, int col, int cnt, const Un
         float qj[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            xj[u] = sx[entry_of(e, u)];
-            qj[u] = P.q[entry_of(e, u)];
+            xj[u] = position_at(sx, entry_of(e, u));
+            qj[u] = P.q[entry_of(e, u) >> 4];
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) dh_pair<ENERGY>(xi, xj[u], qk, qj[u], pc, f, ea);
@@ -862,8 +909,8 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     const float* ginvm = reinterpret_cast<const float*>(blob + R.off_invm);
     const int cls = MODE == kClassGo ? kClassGo : R.cls;
     const bool plain_cls = MODE != kClassGeneral || cls != kClassGeneral;  // Go or Hps
-    const int S = pair_split(n, kSplitUnits), lg = __ffs(S) - 1;
-    const int nq = R.nq, Sq = pair_split(nq, kSplitCharged), lgq = __ffs(Sq) - 1;
+    const int S = pair_split(n, split_units(cls)), lg = __ffs(S) - 1;
+    const int nq = R.nq, Sq = pair_split(nq, charged_units(cls)), lgq = __ffs(Sq) - 1;
     UnitList lm, lq;
     lm.cols = list_columns(n, S);
     lq.cols = list_columns(nq, Sq);
@@ -1175,9 +1222,9 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
                     const float3 g = gaussian3(lc.seed, lc.stream, (uint32_t)b, step, kPurposeLangevin);
                     const float sq = sqrtf(im) * lc.noise;
                     const float fs = lc.fscale * im;
-                    const float vx = lc.vscale * sv[b] + fs * fx + sq * g.x;
-                    const float vy = lc.vscale * sv[ns + b] + fs * fy + sq * g.y;
-                    const float vz = lc.vscale * sv[2 * ns + b] + fs * fz + sq * g.z;
+                    const float vx = __fmaf_rn(fs, fx, __fmaf_rn(lc.vscale, sv[b], sq * g.x));
+                    const float vy = __fmaf_rn(fs, fy, __fmaf_rn(lc.vscale, sv[ns + b], sq * g.y));
+                    const float vz = __fmaf_rn(fs, fz, __fmaf_rn(lc.vscale, sv[2 * ns + b], sq * g.z));
                     sv[b] = vx;
                     sv[ns + b] = vy;
                     sv[2 * ns + b] = vz;
@@ -1657,8 +1704,8 @@ int initial_list_capacity(int64_t m, const uint16_t* idx, int S, double rc, cons
 
 // Entries that a system's two lists take, main first.
 int64_t list_entries(const BatchSys& R) {
-    return (int64_t)R.maxn * list_columns(R.n, pair_split(R.n, kSplitUnits)) +
-           (int64_t)R.maxq * list_columns(R.nq, pair_split(R.nq, kSplitCharged));
+    return (int64_t)R.maxn * list_columns(R.n, pair_split(R.n, split_units(R.cls))) +
+           (int64_t)R.maxq * list_columns(R.nq, pair_split(R.nq, charged_units(R.cls)));
 }
 
 void check_batchable(const CompiledSystem& c, int nmax) {
@@ -1827,8 +1874,8 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
     R.cls = pairs.cls;
     R.n = (int)n;
     R.nq = (int)nq;
-    R.maxn = initial_list_capacity(n, nullptr, pair_split((int)n, kSplitUnits), pairs.main_rc, pos);
-    R.maxq = nq ? initial_list_capacity(nq, pairs.charged.data(), pair_split((int)nq, kSplitCharged), pairs.dh_rc, pos) : 0;
+    R.maxn = initial_list_capacity(n, nullptr, pair_split((int)n, split_units(R.cls)), pairs.main_rc, pos);
+    R.maxq = nq ? initial_list_capacity(nq, pairs.charged.data(), pair_split((int)nq, charged_units(R.cls)), pairs.dh_rc, pos) : 0;
     R.main_rc = (float)pairs.main_rc;
     R.dh_rc = (float)pairs.dh_rc;
     const int64_t boff = beads_.alloc(n, 1);
@@ -2160,8 +2207,8 @@ void BatchEngine::grow_lists() {
         Slot& S = slots_[s];
         BatchSys R = sys_host_[s];
         auto grown = [](int cap, int limit) { return std::min((int)align_up(cap * 3 / 2 + 8, 4), limit); };
-        R.maxn = grown(R.maxn, unit_capacity_limit(R.n, pair_split(R.n, kSplitUnits)));
-        if (R.nq) R.maxq = grown(R.maxq, unit_capacity_limit(R.nq, pair_split(R.nq, kSplitCharged)));
+        R.maxn = grown(R.maxn, unit_capacity_limit(R.n, pair_split(R.n, split_units(R.cls))));
+        if (R.nq) R.maxq = grown(R.maxq, unit_capacity_limit(R.nq, pair_split(R.nq, charged_units(R.cls))));
         const int64_t size = list_entries(R);
         list_alloc_.release(S.list_off, S.list_size);
         const int64_t off = list_alloc_.alloc(size, 64);

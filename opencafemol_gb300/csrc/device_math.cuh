@@ -44,6 +44,14 @@ __device__ __forceinline__ float norm2(float3 d) {
     return __fmaf_rn(d.z, d.z, __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x)));
 }
 
+__device__ __forceinline__ float3 cross3(float3 a, float3 b) {
+    return make_float3(__fmaf_rn(a.y, b.z, -__fmul_rn(a.z, b.y)), __fmaf_rn(a.z, b.x, -__fmul_rn(a.x, b.z)),
+                       __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ float dot3(float3 a, float3 b) {
+    return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
+
 // Label test of an interaction-group matrix: 4-bit label per term, 15 = the
 // particle takes no part in the term.
 __device__ __forceinline__ bool labels_allow(uint32_t li, uint32_t lj, int term,
@@ -231,7 +239,7 @@ __device__ __forceinline__ float ff_bond_delta(float3 dh, float3 dl, float r0sq_
     float t1, t2;
     const float s1 = two_sum(px, py, t1);
     const float s2 = two_sum(s1, pz, t2);
-    const float lo = t1 + t2 + ex + ey + ez + 2.f * (dh.x * dl.x + dh.y * dl.y + dh.z * dl.z);
+    const float lo = __fmaf_rn(2.f, dot3(dh, dl), t1 + t2 + ex + ey + ez);
     return __fsub_rn(s2, r0sq_hi) + (lo - r0sq_lo);
 }
 // Separation x_j - x_i of float-float positions: hi part exact by TwoSum.
@@ -250,15 +258,8 @@ __device__ __forceinline__ void ff_sep(float4 hi_i, float3 lo_i, float4 hi_j, fl
 // E = k (spline(theta) - Emin + step(tmin-theta)(30 (tmin-theta) + y0)
 //                             + step(theta-tmax)(30 (theta-tmax) + y9)),
 // spline = natural cubic spline through 10 equidistant nodes, 0 outside.
-// Writes forces on the three particles.
-__device__ __forceinline__ void fla_forces(float3 u, float3 v, float kk, const FlaTable& t,
-                                           float3& f1, float3& f3, float& energy) {
-    // u = x1 - x2, v = x3 - x2
-    const float3 n = make_float3(u.y * v.z - u.z * v.y, u.z * v.x - u.x * v.z, u.x * v.y - u.y * v.x);
-    const float nn = fmaxf(norm2(n), 1e-30f);
-    const float nlen = sqrtf(nn);
-    const float dot = u.x * v.x + u.y * v.y + u.z * v.z;
-    const float theta = atan2f(nlen, dot);
+// Returns dE/dtheta.
+__device__ __forceinline__ float fla_slope(float theta, float kk, const FlaTable& t, float& energy) {
     float S = 0.f, dS = 0.f;
     if (theta < t.theta_min) {
         S = 30.f * (t.theta_min - theta) + t.y[0];
@@ -273,15 +274,26 @@ __device__ __forceinline__ void fla_forces(float3 u, float3 v, float kk, const F
         const float A = 1.f - B;
         const float yk = t.y[k], yk1 = t.y[k + 1];
         const float mk = t.m[k], mk1 = t.m[k + 1];  // M * h^2 / 6
-        S = A * yk + B * yk1 + (A * A * A - A) * mk + (B * B * B - B) * mk1;
-        dS = ((yk1 - yk) + (1.f - 3.f * A * A) * mk + (3.f * B * B - 1.f) * mk1) * t.inv_h;
+        const float A2 = A * A, B2 = B * B;
+        S = __fmaf_rn(__fmaf_rn(A2, A, -A), mk, __fmaf_rn(__fmaf_rn(B2, B, -B), mk1, __fmaf_rn(A, yk, B * yk1)));
+        dS = __fmaf_rn(__fmaf_rn(-3.f, A2, 1.f), mk, __fmaf_rn(__fmaf_rn(3.f, B2, -1.f), mk1, yk1 - yk)) * t.inv_h;
     }
     energy = kk * (S - t.emin);
-    const float dE = kk * dS;
+    return kk * dS;
+}
+// Writes forces on the first and the last of the three particles.
+__device__ __forceinline__ void fla_forces(float3 u, float3 v, float kk, const FlaTable& t,
+                                           float3& f1, float3& f3, float& energy) {
+    // u = x1 - x2, v = x3 - x2
+    const float3 n = cross3(u, v);
+    const float nn = fmaxf(norm2(n), 1e-30f);
+    const float nlen = sqrtf(nn);
+    const float dot = dot3(u, v);
+    const float dE = fla_slope(atan2f(nlen, dot), kk, t, energy);
     const float uu = norm2(u), vv = norm2(v);
     // dtheta/dx1 = (u x n)/(|u|^2 |n|), dtheta/dx3 = -(v x n)/(|v|^2 |n|)
-    const float3 un = make_float3(u.y * n.z - u.z * n.y, u.z * n.x - u.x * n.z, u.x * n.y - u.y * n.x);
-    const float3 vn = make_float3(v.y * n.z - v.z * n.y, v.z * n.x - v.x * n.z, v.x * n.y - v.y * n.x);
+    const float3 un = cross3(u, n);
+    const float3 vn = cross3(v, n);
     const float c1 = -dE / (uu * nlen);
     const float c3 = dE / (vv * nlen);
     f1 = make_float3(c1 * un.x, c1 * un.y, c1 * un.z);
@@ -296,17 +308,22 @@ struct Torsion {
     float3 A, B;
     float AA, BB, Gl, c, s;
 };
-__device__ __forceinline__ Torsion torsion_geometry(float3 F, float3 G, float3 H) {
+// A = F x G and AA = max(|A|^2, 1e-30) given by the caller.
+__device__ __forceinline__ Torsion torsion_geometry(float3 F, float3 G, float3 H, float3 A, float AA) {
     Torsion t;
-    t.A = make_float3(F.y * G.z - F.z * G.y, F.z * G.x - F.x * G.z, F.x * G.y - F.y * G.x);
-    t.B = make_float3(H.y * G.z - H.z * G.y, H.z * G.x - H.x * G.z, H.x * G.y - H.y * G.x);
-    t.AA = fmaxf(norm2(t.A), 1e-30f);
+    t.A = A;
+    t.B = cross3(H, G);
+    t.AA = AA;
     t.BB = fmaxf(norm2(t.B), 1e-30f);
     t.Gl = sqrtf(norm2(G));
     const float inv_ab = rsqrtf(t.AA * t.BB);
-    t.c = (t.A.x * t.B.x + t.A.y * t.B.y + t.A.z * t.B.z) * inv_ab;
-    t.s = -t.Gl * (F.x * t.B.x + F.y * t.B.y + F.z * t.B.z) * inv_ab;
+    t.c = dot3(t.A, t.B) * inv_ab;
+    t.s = -t.Gl * dot3(F, t.B) * inv_ab;
     return t;
+}
+__device__ __forceinline__ Torsion torsion_geometry(float3 F, float3 G, float3 H) {
+    const float3 A = cross3(F, G);
+    return torsion_geometry(F, G, H, A, fmaxf(norm2(A), 1e-30f));
 }
 // Forces f_a = -dE/dphi * dphi/dx_a.
 __device__ __forceinline__ void torsion_forces(const Torsion& t, float3 F, float3 G, float3 H,
@@ -314,16 +331,17 @@ __device__ __forceinline__ void torsion_forces(const Torsion& t, float3 F, float
                                                float3& f4) {
     const float3 A = t.A, B = t.B;
     const float ga = t.Gl / t.AA, gb = t.Gl / t.BB;
-    const float fg = (F.x * G.x + F.y * G.y + F.z * G.z) / (t.AA * t.Gl);
-    const float hg = (H.x * G.x + H.y * G.y + H.z * G.z) / (t.BB * t.Gl);
+    const float fg = dot3(F, G) / (t.AA * t.Gl);
+    const float hg = dot3(H, G) / (t.BB * t.Gl);
     // dphi/dx1 = -ga A ; dphi/dx4 = gb B
     const float3 d1 = make_float3(-ga * A.x, -ga * A.y, -ga * A.z);
     const float3 d4 = make_float3(gb * B.x, gb * B.y, gb * B.z);
     // dphi/dx2 = ga A + fg A - hg B ; dphi/dx3 = -gb B - fg A + hg B
-    const float3 d2 = make_float3((ga + fg) * A.x - hg * B.x, (ga + fg) * A.y - hg * B.y,
-                                  (ga + fg) * A.z - hg * B.z);
-    const float3 d3 = make_float3(-fg * A.x + (hg - gb) * B.x, -fg * A.y + (hg - gb) * B.y,
-                                  -fg * A.z + (hg - gb) * B.z);
+    const float2 k2 = make_float2(ga + fg, -hg), k3 = make_float2(-fg, hg - gb);
+    const float3 d2 = make_float3(__fmaf_rn(k2.x, A.x, k2.y * B.x), __fmaf_rn(k2.x, A.y, k2.y * B.y),
+                                  __fmaf_rn(k2.x, A.z, k2.y * B.z));
+    const float3 d3 = make_float3(__fmaf_rn(k3.x, A.x, k3.y * B.x), __fmaf_rn(k3.x, A.y, k3.y * B.y),
+                                  __fmaf_rn(k3.x, A.z, k3.y * B.z));
     f1 = make_float3(-dE * d1.x, -dE * d1.y, -dE * d1.z);
     f2 = make_float3(-dE * d2.x, -dE * d2.y, -dE * d2.z);
     f3 = make_float3(-dE * d3.x, -dE * d3.y, -dE * d3.z);
@@ -333,28 +351,28 @@ __device__ __forceinline__ void torsion_forces(const Torsion& t, float3 F, float
 // Flexible-local dihedral (FlexibleLocalDihedralForceFieldGenerator.cpp:7-59):
 // E = k (c - Emin + sum_n a_n cos(n phi) + b_n sin(n phi)), n = 1..3, with
 // the multiple angles from cos/sin recurrences.
-__device__ __forceinline__ void fld_forces(float3 F, float3 G, float3 H, float kk,
+__device__ __forceinline__ void fld_forces(const Torsion& g, float3 F, float3 G, float3 H, float kk,
                                            const FldTable& t, float3& f1, float3& f2,
                                            float3& f3, float3& f4, float& energy) {
-    const Torsion g = torsion_geometry(F, G, H);
     const float c1 = g.c, s1 = g.s;
-    const float c2 = c1 * c1 - s1 * s1, s2 = 2.f * s1 * c1;
-    const float c3 = c1 * c2 - s1 * s2, s3 = s1 * c2 + c1 * s2;
-    energy = kk * (t.c[0] - t.emin + t.c[1] * c1 + t.c[2] * s1 + t.c[3] * c2 + t.c[4] * s2 +
-                   t.c[5] * c3 + t.c[6] * s3);
-    const float dE = kk * (-t.c[1] * s1 + t.c[2] * c1 - 2.f * t.c[3] * s2 + 2.f * t.c[4] * c2 -
-                           3.f * t.c[5] * s3 + 3.f * t.c[6] * c3);
+    const float c2 = __fmaf_rn(c1, c1, -(s1 * s1)), s2 = 2.f * s1 * c1;
+    const float c3 = __fmaf_rn(c1, c2, -(s1 * s2)), s3 = __fmaf_rn(s1, c2, c1 * s2);
+    energy = kk * __fmaf_rn(t.c[6], s3, __fmaf_rn(t.c[5], c3, __fmaf_rn(t.c[4], s2, __fmaf_rn(t.c[3], c2,
+                  __fmaf_rn(t.c[2], s1, __fmaf_rn(t.c[1], c1, t.c[0] - t.emin))))));
+    const float e1 = __fmaf_rn(t.c[2], c1, -(t.c[1] * s1));
+    const float e2 = __fmaf_rn(t.c[4], c2, -(t.c[3] * s2));
+    const float e3 = __fmaf_rn(t.c[6], c3, -(t.c[5] * s3));
+    const float dE = kk * __fmaf_rn(3.f, e3, __fmaf_rn(2.f, e2, e1));
     torsion_forces(g, F, G, H, dE, f1, f2, f3, f4);
 }
 
 // Gaussian dihedral (GaussianDihedralForceFieldGenerator.cpp:5-12):
 // E = k exp(-dp^2 / (2 sigma^2)), dp = d - floor((d + pi) / (2 pi)) 2 pi,
 // d = phi - theta0; inv2s2 = 1 / (2 sigma^2).
-__device__ __forceinline__ void gauss_dihedral_forces(float3 F, float3 G, float3 H, float kk,
-                                                      float theta0, float inv2s2, float3& f1,
+__device__ __forceinline__ void gauss_dihedral_forces(const Torsion& g, float3 F, float3 G, float3 H,
+                                                      float kk, float theta0, float inv2s2, float3& f1,
                                                       float3& f2, float3& f3, float3& f4,
                                                       float& energy) {
-    const Torsion g = torsion_geometry(F, G, H);
     const float phi = atan2f(g.s, g.c);
     const float two_pi = 6.2831853071795865f;
     float d = phi - theta0;

@@ -918,11 +918,12 @@ __global__ void __launch_bounds__(kForceThreads) k_forces(ForceArgs a) {
                 const float3 H = bonded_sep(a, q.k, q.l, q.periodic);  // x4 - x3
                 float3 f1, f2, f3, f4;
                 float en;
+                const Torsion g = torsion_geometry(F, G, H);
                 if (q.kind == kDihFLD) {
-                    fld_forces(F, G, H, q.kk, a.fld[q.table], f1, f2, f3, f4, en);
+                    fld_forces(g, F, G, H, q.kk, a.fld[q.table], f1, f2, f3, f4, en);
                     efld = en;
                 } else {
-                    gauss_dihedral_forces(F, G, H, q.kk, q.theta0, q.inv2s2, f1, f2, f3, f4, en);
+                    gauss_dihedral_forces(g, F, G, H, q.kk, q.theta0, q.inv2s2, f1, f2, f3, f4, en);
                     egd = en;
                 }
                 add_force(a, q.i, f1);

@@ -57,7 +57,28 @@ struct ListFlags {
     // kBlownUp: a force contribution or a summed force of 1e9 kJ/mol/nm or
     // more (the fixed-point accumulators hold about 2.1e9), a non-finite
     // force, velocity or position
-    enum : int { kTileOverflow = 1, kMaskOverflow = 2, kSkinViolation = 4, kChargedOverflow = 8, kBlownUp = 16 };
+    enum : int {
+        kTileOverflow = 1,
+        kMaskOverflow = 2,
+        kSkinViolation = 4,
+        kChargedOverflow = 8,
+        kBlownUp = 16,
+        kListOverflow = 32,
+        kNeighbourOverflow = 64
+    };
+};
+
+// Per-bead pair lists over staged neighbour clusters (plain path).
+struct NeighbourLists {
+    int cap;          // neighbour clusters per cluster
+    int list_groups;  // groups of four entries per unit
+    int32_t *cnt, *j; // neighbour clusters of every cluster
+    float4* shift;    // their anchor shifts, w != 0: minimum image needed
+    int32_t* len;     // list entries of every bead (cluster slot)
+    uint16_t* list;
+    float4* ljs;      // cluster order: half sigma, half epsilon (repulsive, attractive), half attractive sigma
+    int32_t* stats;   // most neighbours of a cluster, longest unit, neighbour pairs
+    int32_t* flags;
 };
 
 class BatchEngine;
@@ -116,6 +137,13 @@ class PlainContext {
     void ensure_capacity();
     cudaGraphExec_t graph_for(int chunk);
     void clear_graphs();
+    void rebuild_pair_lists(cudaStream_t s, float cut);
+    void rebuild_charged_rows(cudaStream_t s);
+    NeighbourLists neighbour_lists() const;
+    size_t list_smem(bool same_sigma, bool build) const;
+    int column_reach(float cut, int reach[2]) const;
+    void alloc_pair_lists();
+    void leave_pair_lists();
     void setup_charged_cells();
     void setup_columns(double width);
     BoxD box_d() const;
@@ -157,6 +185,13 @@ class PlainContext {
     int charged_cells_[3] = {1, 1, 1};
     int64_t n_charged_ = 0, n_charged_cells_ = 0, charged_last_ = 0;
     int64_t chg_row_cap_ = 0;  // entries per charged bead's row
+
+    // Per-bead pair lists of the Lennard-Jones terms instead of tiles
+    bool pair_lists_ = false;
+    int nbr_cap_ = 0, list_cap_ = 0;  // neighbour clusters per cluster, entries per unit
+    DevBuf<int32_t> nbr_cnt_, nbr_j_, list_len_, nbr_stats_;
+    DevBuf<float4> nbr_shift_, ljs_;
+    DevBuf<uint16_t> list_;
 
     // per particle (original order)
     DevBuf<double> x_, y_, z_;

@@ -242,7 +242,8 @@ __global__ void k_gather_sorted(int np, const int32_t* __restrict__ perm,
                                 int32_t* __restrict__ slot, float4* __restrict__ xs,
                                 float4* __restrict__ anc,
                                 float4* __restrict__ p0s, float4* __restrict__ p1s,
-                                uint32_t* __restrict__ labs, float4* __restrict__ ref) {
+                                uint32_t* __restrict__ labs, float4* __restrict__ ref,
+                                float4* __restrict__ ljs) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= np) return;
     const int o = perm[k];
@@ -263,11 +264,13 @@ __global__ void k_gather_sorted(int np, const int32_t* __restrict__ perm,
         p0s[k] = p0[o];
         p1s[k] = p1[o];
         labs[k] = lab[o];
+        if (ljs) ljs[k] = make_float4(0.5f * p0[o].w, 0.5f * p0[o].z, 0.5f * p1[o].x, 0.5f * p1[o].y);
     } else {
         xs[k] = make_float4(nan, nan, nan, 0.f);
         p0s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         p1s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         labs[k] = 0xffffffffu;
+        if (ljs) ljs[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -658,6 +661,230 @@ __global__ void k_chg_list_pairs(int m, const int32_t* __restrict__ idx, const i
 }
 
 // ---------------------------------------------------------------------------
+// Per-bead pair lists (the Lennard-Jones terms of large periodic systems).
+// A force block owns one cluster: it stages the positions of every neighbour
+// cluster in shared memory and walks each bead's list of its partners among
+// them, both directions of a pair, so the pair forces need no atomics but one
+// per bead and component.  A unit is a bead and every kListUnits-th of its
+// partners (adjacent lanes share a bead); a unit's entries are 8 x the staged
+// slot, in groups of four, the groups of a cluster's units side by side; the
+// last group is filled up with the dummy bead behind the staged ones.
+// ---------------------------------------------------------------------------
+constexpr int kMaxNeighbours = 128;  // so that an entry fits 16 bits
+constexpr int kMaxColumns = 512;     // columns a neighbourhood may span
+constexpr int kMaxCandidates = 512;  // clusters whose boxes are in reach
+constexpr int kListUnits = 8;
+constexpr int kListThreads = 32 * kListUnits;
+constexpr int kBuildThreads = 512;
+constexpr int kBuildWarps = kBuildThreads / 32;
+
+__device__ __forceinline__ size_t list_at(const NeighbourLists& nb, int I, int k, int unit) {
+    return (((size_t)I * nb.list_groups + (k >> 2)) * kListThreads + unit) * 4 + (k & 3);
+}
+// Entries of unit s of a bead with len partners.
+__device__ __forceinline__ int unit_entries(int len, int s) { return (len - s + kListUnits - 1) / kListUnits; }
+
+// Neighbour clusters and lists of every cluster, one block each.
+//  1. The clusters of the columns within reach whose bounding boxes are
+//     within the cutoff (one warp per column: a count pass, then the same
+//     again to write them in column order).
+//  2. Of these, the ones where some bead of either is within the cutoff of
+//     the other's box (one warp each), in order, with their anchor shift and
+//     whether their pairs need the minimum image (see k_compact_tiles).
+//  3. One warp per bead: the lanes test the neighbour boxes, then 32 staged
+//     beads of each box that is near; hits are compacted by ballot.  A list
+//     holds the partners within cut (the canonical separation of the force
+//     kernel) that the exclusions keep, in neighbour order.
+// Columns within reach, not all clusters, and the two bead tests take the
+// place of the tiles' sweep over every cluster, exact pruning and exclusion
+// masks (eight launches).
+__global__ void __launch_bounds__(kBuildThreads, 2)
+    k_pair_lists(int nc, int nx, int ny, int nz, int rx, int ry, const int32_t* __restrict__ perm,
+                 const int32_t* __restrict__ key, const int32_t* __restrict__ col_start,
+                 const int32_t* __restrict__ slot, const float4* __restrict__ xs, const float4* __restrict__ bc,
+                 const float4* __restrict__ bh, const float4* __restrict__ ext, BoxD bd, float3 box, float3 inv_box,
+                 float pad, float cut, const int32_t* __restrict__ ex_csr, const int32_t* __restrict__ ex_j,
+                 const uint8_t* __restrict__ ex_bits, NeighbourLists nb) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float4* px = reinterpret_cast<float4*>(smem);
+    float4* sA = px + 32 * nb.cap + 1;
+    __shared__ int s_col[kMaxColumns + 1];
+    __shared__ int s_cand[kMaxCandidates];
+    __shared__ unsigned char s_keep[kMaxCandidates];
+    __shared__ int sj[kMaxNeighbours];
+    __shared__ int s_m;
+    const int I = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float4 hi = bh[I];
+    if (hi.w < 0.f) {  // padding slots only
+        if (tid == 0) nb.cnt[I] = 0;
+        return;
+    }
+    const float cut2 = cut * cut;
+    const float4 ci = bc[I];
+    const int col = key[perm[I * 32]] / nz, cx = col % nx, cy = col / nx;
+    const bool all_x = 2 * rx + 1 >= nx, all_y = 2 * ry + 1 >= ny;
+    const int wx = all_x ? nx : 2 * rx + 1, columns = wx * (all_y ? ny : 2 * ry + 1);
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int v = warp; v < columns; v += kBuildWarps) {
+            const int ix = v % wx, iy = v / wx;
+            const int x = all_x ? ix : (cx - rx + ix + nx) % nx, y = all_y ? iy : (cy - ry + iy + ny) % ny;
+            const int q0 = col_start[y * nx + x] >> 5, q1 = col_start[y * nx + x + 1] >> 5;
+            int at = pass ? s_col[v] : 0;
+            for (int J = q0 + lane; J - lane < q1; J += 32) {
+                bool ok = false;
+                if (J < q1) {
+                    const float4 hj = bh[J];
+                    ok = hj.w >= 0.f && boxes_close<true>(ci, hi, bc[J], hj, box, inv_box, cut, cut2);
+                }
+                const unsigned bal = __ballot_sync(kFull, ok);
+                const int to = at + __popc(bal & ((1u << lane) - 1u));
+                if (pass && ok && to < kMaxCandidates) s_cand[to] = J;
+                at += __popc(bal);
+            }
+            if (!pass && lane == 0) s_col[v] = at;
+        }
+        __syncthreads();
+        if (!pass) {
+            if (warp == 0) {  // exclusive scan of the columns' counts
+                int run = 0;
+                for (int v0 = 0; v0 < columns; v0 += 32) {
+                    const int c = v0 + lane < columns ? s_col[v0 + lane] : 0;
+                    int incl = c;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int u = __shfl_up_sync(kFull, incl, o);
+                        if (lane >= o) incl += u;
+                    }
+                    if (v0 + lane < columns) s_col[v0 + lane] = run + incl - c;
+                    run += __shfl_sync(kFull, incl, 31);
+                }
+                if (lane == 0) s_col[columns] = run;
+            }
+            __syncthreads();
+        }
+    }
+    const int cands = min(s_col[columns], kMaxCandidates);
+    {
+        const float4 xi = xs[I * 32 + lane];
+        for (int c = warp; c < cands; c += kBuildWarps) {
+            const int J = s_cand[c];
+            const float4 cj = bc[J], hj = bh[J], xj = xs[J * 32 + lane];
+            const float3 d = min_image(make_float3(cj.x - ci.x, cj.y - ci.y, cj.z - ci.z), box, inv_box);
+            auto near = [&](float4 x, float sign, float4 h) {  // false for padding (NaN)
+                const float gx = fmaxf(0.f, fabsf(d.x + sign * x.x) - h.x);
+                const float gy = fmaxf(0.f, fabsf(d.y + sign * x.y) - h.y);
+                const float gz = fmaxf(0.f, fabsf(d.z + sign * x.z) - h.z);
+                return x.x == x.x && gx * gx + gy * gy + gz * gz < cut2;
+            };
+            const bool wide = hi.x + hj.x + cut >= 0.5f * box.x || hi.y + hj.y + cut >= 0.5f * box.y ||
+                              hi.z + hj.z + cut >= 0.5f * box.z;
+            const bool keep = wide || (__any_sync(kFull, near(xi, -1.f, hj)) && __any_sync(kFull, near(xj, 1.f, hi)));
+            if (lane == 0) s_keep[c] = keep;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        int m = 0, upper = 0;
+        const float4 ei = ext[I];
+        for (int c0 = 0; c0 < cands; c0 += 32) {
+            const bool keep = c0 + lane < cands && s_keep[c0 + lane];
+            const unsigned bal = __ballot_sync(kFull, keep);
+            const int to = m + __popc(bal & ((1u << lane) - 1u));
+            const int J = keep ? s_cand[c0 + lane] : I;
+            if (keep && to < nb.cap) {
+                const float3 A = anchor_shift(ci, bc[J], bd);
+                const float4 ej = ext[J];
+                const bool wrap = fabsf(A.x) + ei.x + ej.x + pad >= 0.5f * box.x ||
+                                  fabsf(A.y) + ei.y + ej.y + pad >= 0.5f * box.y ||
+                                  fabsf(A.z) + ei.z + ej.z + pad >= 0.5f * box.z;
+                const float4 shift = make_float4(A.x, A.y, A.z, wrap ? 1.f : 0.f);
+                sj[to] = J;
+                sA[to] = shift;
+                nb.j[(size_t)I * nb.cap + to] = J;
+                nb.shift[(size_t)I * nb.cap + to] = shift;
+            }
+            upper += __popc(__ballot_sync(kFull, keep && J >= I));
+            m += __popc(bal);
+        }
+        if (lane == 0) {
+            s_m = min(m, nb.cap);
+            nb.cnt[I] = min(m, nb.cap);
+            atomicMax(&nb.stats[0], s_col[columns] > kMaxCandidates ? kMaxNeighbours + 1 : m);
+            atomicAdd(&nb.stats[2], upper);
+            if (m > nb.cap || s_col[columns] > kMaxCandidates) atomicOr(nb.flags, ListFlags::kNeighbourOverflow);
+        }
+    }
+    __syncthreads();
+    const int m = s_m;
+    for (int t = tid; t < 32 * m; t += kBuildThreads) px[t] = xs[sj[t >> 5] * 32 + (t & 31)];
+    __syncthreads();
+    const int unit_cap = nb.list_groups * 4;
+    for (int b = warp; b < 32; b += kBuildWarps) {
+        const int o = perm[I * 32 + b];
+        if (o < 0) {
+            if (lane == 0) nb.len[I * 32 + b] = 0;
+            continue;
+        }
+        const int e0 = ex_csr[o], e1 = ex_csr[o + 1];
+        auto excluded_slot = [&](int e) { return e < e1 && (ex_bits[e] & kTermLJR) ? slot[ex_j[e]] : -1; };
+        const int first = excluded_slot(e0 + lane);
+        const bool many = e1 - e0 > 32;
+        const float4 xi = xs[I * 32 + b];
+        int cnt = 0;
+        for (int h = 0; h < m; h += 32) {
+            bool ok = false;
+            const int Jh = h + lane < m ? sj[h + lane] : -1;
+            if (Jh >= 0) {
+                const float4 A = sA[h + lane], hj = bh[Jh];
+                const float gx = fmaxf(0.f, fabsf(A.x - xi.x) - hj.x);
+                const float gy = fmaxf(0.f, fabsf(A.y - xi.y) - hj.y);
+                const float gz = fmaxf(0.f, fabsf(A.z - xi.z) - hj.z);
+                ok = A.w != 0.f || gx * gx + gy * gy + gz * gz < cut2;
+            }
+            // boxes that hold an excluded partner (every box when the row is long)
+            bool holds = many;
+            if (!many)
+                for (int e = 0; e < e1 - e0; ++e) {
+                    const int x = __shfl_sync(kFull, first, e);
+                    holds = holds || (x >= 0 && x >> 5 == Jh);
+                }
+            const unsigned hold_mask = __ballot_sync(kFull, holds);
+            for (unsigned left = __ballot_sync(kFull, ok); left; left &= left - 1) {
+                const int l = __ffs(left) - 1, q = h + l;
+                const float4 A = sA[q];
+                float3 d = anchored_sep(xi, px[32 * q + lane], make_float3(A.x, A.y, A.z));
+                if (A.w != 0.f) d = min_image(d, box, inv_box);
+                unsigned hits = __ballot_sync(kFull, norm2(d) < cut2);
+                const int J = sj[q];
+                if (J == I) hits &= ~(1u << b);
+                if (hold_mask >> l & 1u)
+                    for (int e = e0; e < e1; e += 32) {
+                        const int ex = e == e0 ? first : excluded_slot(e + lane);
+                        for (unsigned x = __ballot_sync(kFull, ex >= 0 && ex >> 5 == J); x; x &= x - 1)
+                            hits &= ~(1u << (__shfl_sync(kFull, ex, __ffs(x) - 1) & 31));
+                    }
+                if (hits >> lane & 1u) {
+                    const int k = cnt + __popc(hits & ((1u << lane) - 1u));
+                    if (k / kListUnits < unit_cap)
+                        nb.list[list_at(nb, I, k / kListUnits, kListUnits * b + k % kListUnits)] =
+                            (uint16_t)((32 * q + lane) << 3);
+                }
+                cnt += __popc(hits);
+            }
+        }
+        if (lane < kListUnits)  // fill up the unit's last group
+            for (int k = unit_entries(cnt, lane); (k & 3) && k < unit_cap; ++k)
+                nb.list[list_at(nb, I, k, kListUnits * b + lane)] = (uint16_t)((32 * nb.cap) << 3);
+        if (lane == 0) {
+            const int longest = unit_entries(cnt, 0);
+            nb.len[I * 32 + b] = min(cnt, kListUnits * unit_cap);
+            if (longest > unit_cap) atomicOr(nb.flags, ListFlags::kListOverflow);
+            atomicMax(&nb.stats[1], longest);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Fused force kernel
 // ---------------------------------------------------------------------------
 struct ForceArgs {
@@ -682,6 +909,7 @@ struct ForceArgs {
     uint32_t excl_all;
     double* energy;
     const float4* tile_shift;  // per tile: anchor shift a_J - a_I, w != 0: minimum image needed
+    NeighbourLists nb;         // per-bead pair lists (k_forces_lists)
     // charged-pair rows (blocks_chg > 0)
     const float4 *xq, *xlo, *p0;
     const int32_t *chg_idx, *chg_rows, *chg_len;
@@ -715,6 +943,159 @@ __device__ __forceinline__ float3 bonded_sep(const ForceArgs& a, int i, int j, i
         d.z -= a.box.z * rintf(d.z * a.inv_box.z);
     }
     return d;
+}
+
+// Bonded terms and charged rows: the segments behind the pair blocks.
+template <bool PERIODIC, bool ENERGY, int THREADS>
+__device__ __forceinline__ void other_segments(const ForceArgs& a, int blk) {
+    const int lane = threadIdx.x & 31;
+    if (blk < a.blocks_bonds) {
+        // ------------ harmonic bonds, Go contacts, Gaussian bonds ------------
+        const int t = blk * THREADS + threadIdx.x;
+        float eh = 0.f, eg = 0.f, eb = 0.f, ec = 0.f;
+        if (t < a.n_bonds) {
+            const BondTerm b = a.bonds[t];
+            const int slot = bond_slot(b.kind);
+            if (a.slots_enabled & (1u << slot)) {
+                double dx = a.x[b.j] - a.x[b.i], dy = a.y[b.j] - a.y[b.i], dz = a.z[b.j] - a.z[b.i];
+                if (b.periodic) {
+                    dx -= (double)a.box.x * rint(dx * (double)a.inv_box.x);
+                    dy -= (double)a.box.y * rint(dy * (double)a.inv_box.y);
+                    dz -= (double)a.box.z * rint(dz * (double)a.inv_box.z);
+                }
+                const double r2d = dx * dx + dy * dy + dz * dz;
+                const float delta = (float)(r2d - ((double)b.r0sq_hi + (double)b.r0sq_lo));
+                const float3 d = make_float3((float)dx, (float)dy, (float)dz);
+                float en;
+                const float s = bond_scalar(b.kind, norm2(d), delta, b.p0, b.p1, b.r0sq_hi, en);
+                add_force(a, b.i, make_float3(-s * d.x, -s * d.y, -s * d.z));
+                add_force(a, b.j, make_float3(s * d.x, s * d.y, s * d.z));
+                if (b.kind == kBondHarmonic) eh = en;
+                else if (b.kind == kBondGo) eg = en;
+                else if (b.kind == kBondGauss) eb = en;
+                else ec = en;
+            }
+        }
+        if (ENERGY) {
+            const double vh = warp_sum((double)eh), vg = warp_sum((double)eg), vb = warp_sum((double)eb),
+                         vc = warp_sum((double)ec);
+            if (lane == 0) {
+                if (vh != 0.0) atomicAdd(&a.energy[kSlotHB], vh);
+                if (vg != 0.0) atomicAdd(&a.energy[kSlotGO], vg);
+                if (vb != 0.0) atomicAdd(&a.energy[kSlotGB], vb);
+                if (vc != 0.0) atomicAdd(&a.energy[kSlotCGO], vc);
+            }
+        }
+        return;
+    }
+    blk -= a.blocks_bonds;
+    if (blk < a.blocks_angles) {
+        const int t = blk * THREADS + threadIdx.x;
+        float en = 0.f;
+        if (t < a.n_angles && (a.slots_enabled & (1u << kSlotFLA))) {
+            const AngleTerm g = a.angles[t];
+            const float3 u = bonded_sep(a, g.j, g.i, g.periodic);  // x1 - x2
+            const float3 v = bonded_sep(a, g.j, g.k, g.periodic);  // x3 - x2
+            float3 f1, f3;
+            fla_forces(u, v, g.kk, a.fla[g.table], f1, f3, en);
+            add_force(a, g.i, f1);
+            add_force(a, g.k, f3);
+            add_force(a, g.j, make_float3(-f1.x - f3.x, -f1.y - f3.y, -f1.z - f3.z));
+        }
+        if (ENERGY) {
+            const double v = warp_sum((double)en);
+            if (lane == 0 && v != 0.0) atomicAdd(&a.energy[kSlotFLA], v);
+        }
+        return;
+    }
+    blk -= a.blocks_angles;
+    if (blk < a.blocks_dih) {
+        const int t = blk * THREADS + threadIdx.x;
+        float efld = 0.f, egd = 0.f;
+        if (t < a.n_dih) {
+            const DihedralTerm q = a.dih[t];
+            const int slot = q.kind == kDihFLD ? kSlotFLD : kSlotGD;
+            if (a.slots_enabled & (1u << slot)) {
+                const float3 F = bonded_sep(a, q.j, q.i, q.periodic);  // x1 - x2
+                const float3 G = bonded_sep(a, q.k, q.j, q.periodic);  // x2 - x3
+                const float3 H = bonded_sep(a, q.k, q.l, q.periodic);  // x4 - x3
+                float3 f1, f2, f3, f4;
+                float en;
+                const Torsion g = torsion_geometry(F, G, H);
+                if (q.kind == kDihFLD) {
+                    fld_forces(g, F, G, H, q.kk, a.fld[q.table], f1, f2, f3, f4, en);
+                    efld = en;
+                } else {
+                    gauss_dihedral_forces(g, F, G, H, q.kk, q.theta0, q.inv2s2, f1, f2, f3, f4, en);
+                    egd = en;
+                }
+                add_force(a, q.i, f1);
+                add_force(a, q.j, f2);
+                add_force(a, q.k, f3);
+                add_force(a, q.l, f4);
+            }
+        }
+        if (ENERGY) {
+            const double v = warp_sum((double)efld), vg = warp_sum((double)egd);
+            if (lane == 0) {
+                if (v != 0.0) atomicAdd(&a.energy[kSlotFLD], v);
+                if (vg != 0.0) atomicAdd(&a.energy[kSlotGD], vg);
+            }
+        }
+        return;
+    }
+    blk -= a.blocks_dih;
+    {
+        // ---------------- charged pairs (Debye-Hueckel) ----------------
+        // One warp per charged bead over its row; each pair's force on bead
+        // i is rounded to fixed point and summed as integers, then added
+        // once per bead.
+        const int warp = threadIdx.x >> 5;
+        float edh = 0.f;
+        if (a.slots_enabled & (1u << kSlotDH)) {
+            const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int t = blk * (THREADS / 32) + warp; t < a.n_chg; t += a.blocks_chg * (THREADS / 32)) {
+                const int i = a.chg_idx[t];
+                const float4 xi = a.xq[i], li = a.xlo[i];
+                const float4 pi = a.p0[i];
+                const int len = min(a.chg_len[t], a.chg_row_cap);
+                const int32_t* row = a.chg_rows + (size_t)t * a.chg_row_cap;
+                long long fx = 0, fy = 0, fz = 0;
+                bool bad = false;
+                for (int p = lane; p < len; p += 32) {
+                    const int j = row[p];
+                    const float3 d = ff_separation<PERIODIC>(xi, li, a.xq[j], a.xlo[j], a.box, a.inv_box);
+                    const float r2 = norm2(d);
+                    if (r2 < a.pc.dh_rc2) {
+                        PairEnergy e;
+                        e.zero();
+                        const float sc = pair_scalar<kTermDH, ENERGY>(r2, pi, a.p0[j], zero4, zero4, 0u, a.pc, e);
+                        bad = bad || !force_ok(make_float3(sc * d.x, sc * d.y, sc * d.z));
+                        fx += (long long)to_fixed(-sc * d.x);
+                        fy += (long long)to_fixed(-sc * d.y);
+                        fz += (long long)to_fixed(-sc * d.z);
+                        if (ENERGY && i < j) edh += e.dh;
+                    }
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    fx += __shfl_xor_sync(0xffffffffu, fx, o);
+                    fy += __shfl_xor_sync(0xffffffffu, fy, o);
+                    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+                }
+                if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, ListFlags::kBlownUp);
+                if (lane == 0) {
+                    if (fx) atomicAdd(&a.F[i], (unsigned long long)fx);
+                    if (fy) atomicAdd(&a.F[a.n + i], (unsigned long long)fy);
+                    if (fz) atomicAdd(&a.F[2 * a.n + i], (unsigned long long)fz);
+                }
+            }
+        }
+        if (ENERGY) {
+            const double v = warp_sum((double)edh);
+            if (lane == 0 && v != 0.0) atomicAdd(&a.energy[kSlotDH], v);
+        }
+    }
 }
 
 template <int TERMS, bool PERIODIC, bool ENERGY>
@@ -845,152 +1226,160 @@ __global__ void __launch_bounds__(kForceThreads) k_forces(ForceArgs a) {
         }
         return;
     }
-    blk -= a.blocks_tiles;
-    if (blk < a.blocks_bonds) {
-        // ------------ harmonic bonds, Go contacts, Gaussian bonds ------------
-        const int t = blk * kForceThreads + threadIdx.x;
-        float eh = 0.f, eg = 0.f, eb = 0.f, ec = 0.f;
-        if (t < a.n_bonds) {
-            const BondTerm b = a.bonds[t];
-            const int slot = bond_slot(b.kind);
-            if (a.slots_enabled & (1u << slot)) {
-                double dx = a.x[b.j] - a.x[b.i], dy = a.y[b.j] - a.y[b.i], dz = a.z[b.j] - a.z[b.i];
-                if (b.periodic) {
-                    dx -= (double)a.box.x * rint(dx * (double)a.inv_box.x);
-                    dy -= (double)a.box.y * rint(dy * (double)a.inv_box.y);
-                    dz -= (double)a.box.z * rint(dz * (double)a.inv_box.z);
-                }
-                const double r2d = dx * dx + dy * dy + dz * dz;
-                const float delta = (float)(r2d - ((double)b.r0sq_hi + (double)b.r0sq_lo));
-                const float3 d = make_float3((float)dx, (float)dy, (float)dz);
-                float en;
-                const float s = bond_scalar(b.kind, norm2(d), delta, b.p0, b.p1, b.r0sq_hi, en);
-                add_force(a, b.i, make_float3(-s * d.x, -s * d.y, -s * d.z));
-                add_force(a, b.j, make_float3(s * d.x, s * d.y, s * d.z));
-                if (b.kind == kBondHarmonic) eh = en;
-                else if (b.kind == kBondGo) eg = en;
-                else if (b.kind == kBondGauss) eb = en;
-                else ec = en;
-            }
-        }
-        if (ENERGY) {
-            const double vh = warp_sum((double)eh), vg = warp_sum((double)eg), vb = warp_sum((double)eb),
-                         vc = warp_sum((double)ec);
-            if (lane == 0) {
-                if (vh != 0.0) atomicAdd(&a.energy[kSlotHB], vh);
-                if (vg != 0.0) atomicAdd(&a.energy[kSlotGO], vg);
-                if (vb != 0.0) atomicAdd(&a.energy[kSlotGB], vb);
-                if (vc != 0.0) atomicAdd(&a.energy[kSlotCGO], vc);
-            }
-        }
+    other_segments<PERIODIC, ENERGY, kForceThreads>(a, blk - a.blocks_tiles);
+}
+
+// Both Lennard-Jones terms of one pair at separation d; le: half epsilons
+// (repulsive, attractive) and, unless SAME, half the attractive sigma.
+// Inside its core (r <= 2^(1/6) sigma) a term's repulsive part acts and its
+// attractive part is flat; outside it the attractive part acts alone.  With
+// one sigma for both terms (SAME) one power form serves both, with the bits
+// of the general form.  Every operation is rounded by itself.
+template <bool SAME, bool ENERGY>
+__device__ __forceinline__ void lj_pair(float3 d, float hi, float hj, float4 lei, float4 lej, const PairConsts& pc,
+                                        float3& f, float& er_sum, float& ea_sum) {
+    const float r2 = norm2(d);
+    const bool in_r = r2 < pc.ljr_rc2, in_a = SAME ? in_r : r2 < pc.lja_rc2;
+    const float rinv = rsqrtf(r2);
+    const float ri = __fmul_rn(rinv, rinv);
+    const float er = __fadd_rn(lei.x, lej.x), el = __fadd_rn(lei.y, lej.y);
+    auto powers = [&](float sg, float& s6, float& s12, bool& core) {
+        const float sig2 = __fmul_rn(sg, sg);
+        const float s2 = __fmul_rn(sig2, ri);
+        s6 = __fmul_rn(__fmul_rn(s2, s2), s2);
+        s12 = __fmul_rn(s6, s6);
+        core = r2 <= __fmul_rn(sig2, kTwoPow1_3);
+        return __fmul_rn(__fmul_rn(24.f, ri), __fmaf_rn(2.f, s12, -s6));
+    };
+    float s6, s12, a6, a12, ta;
+    bool core, acore;
+    const float t = powers(__fadd_rn(hi, hj), s6, s12, core);
+    if (SAME) {
+        a6 = s6;
+        a12 = s12;
+        acore = core;
+        ta = t;
+    } else {
+        ta = powers(__fadd_rn(lei.z, lej.z), a6, a12, acore);
+    }
+    float rep = core ? __fmul_rn(er, t) : 0.f;
+    float att = acore ? 0.f : __fmul_rn(el, ta);
+    const float r = __fmul_rn(r2, rinv);
+    float sw = 1.f;
+    if (r > pc.lja_rs) {
+        // OpenMM switching function S = 1 - 10x^3 + 15x^4 - 6x^5.
+        const float x = __fmul_rn(__fsub_rn(r, pc.lja_rs), pc.lja_inv_width);
+        const float x2 = __fmul_rn(x, x);
+        const float x3 = __fmul_rn(x2, x);
+        sw = __fmaf_rn(x3, __fmaf_rn(x, __fmaf_rn(-6.f, x, 15.f), -10.f), 1.f);
+        const float dsw = __fmul_rn(__fmul_rn(x2, __fmaf_rn(x, __fmaf_rn(-30.f, x, 60.f), -30.f)), pc.lja_inv_width);
+        const float E = acore ? -el : __fmul_rn(__fmul_rn(4.f, el), __fsub_rn(a12, a6));
+        att = __fmaf_rn(att, sw, -__fmul_rn(__fmul_rn(E, dsw), rinv));
+    }
+    rep = in_r ? rep : 0.f;
+    att = in_a ? att : 0.f;
+    const float s = __fadd_rn(rep, att);
+    f.x = __fmaf_rn(-s, d.x, f.x);
+    f.y = __fmaf_rn(-s, d.y, f.y);
+    f.z = __fmaf_rn(-s, d.z, f.z);
+    if (ENERGY) {
+        if (in_r && core) er_sum += er * (4.f * (s12 - s6) + 1.f);
+        if (in_a) ea_sum += (acore ? -el : el * (4.f * (a12 - a6))) * sw;
+    }
+}
+
+// The force kernel on pair lists: one block per cluster, then the other
+// segments.
+template <bool SAME, bool ENERGY>
+__global__ void __launch_bounds__(kListThreads, 4) k_forces_lists(ForceArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x >= a.blocks_tiles) {
+        other_segments<true, ENERGY, kListThreads>(a, (int)blockIdx.x - a.blocks_tiles);
         return;
     }
-    blk -= a.blocks_bonds;
-    if (blk < a.blocks_angles) {
-        const int t = blk * kForceThreads + threadIdx.x;
-        float en = 0.f;
-        if (t < a.n_angles && (a.slots_enabled & (1u << kSlotFLA))) {
-            const AngleTerm g = a.angles[t];
-            const float3 u = bonded_sep(a, g.j, g.i, g.periodic);  // x1 - x2
-            const float3 v = bonded_sep(a, g.j, g.k, g.periodic);  // x3 - x2
-            float3 f1, f3;
-            fla_forces(u, v, g.kk, a.fla[g.table], f1, f3, en);
-            add_force(a, g.i, f1);
-            add_force(a, g.k, f3);
-            add_force(a, g.j, make_float3(-f1.x - f3.x, -f1.y - f3.y, -f1.z - f3.z));
-        }
-        if (ENERGY) {
-            const double v = warp_sum((double)en);
-            if (lane == 0 && v != 0.0) atomicAdd(&a.energy[kSlotFLA], v);
-        }
-        return;
+    const NeighbourLists& nb = a.nb;
+    const int I = blockIdx.x;
+    const int m = nb.cnt[I];
+    if (m == 0) return;  // padding slots only
+    const int dummy = 32 * nb.cap;
+    float4* px = reinterpret_cast<float4*>(smem);
+    float4* sA = px + dummy + 1;
+    unsigned char* sle = reinterpret_cast<unsigned char*>(sA + nb.cap + 1);
+    float2* le2 = reinterpret_cast<float2*>(sle);
+    float4* le4 = reinterpret_cast<float4*>(sle);
+    const int k = I * 32 + tid / kListUnits;  // this unit's bead
+    const int groups = (unit_entries(nb.len[k], tid % kListUnits) + 3) >> 2;
+    const uint2* list = reinterpret_cast<const uint2*>(nb.list) + (size_t)I * nb.list_groups * kListThreads + tid;
+    uint2 e = groups > 0 ? list[0] : make_uint2(0u, 0u);
+    const float er_on = a.excl_all & kTermLJR ? 0.f : 1.f, ea_on = a.excl_all & kTermLJA ? 0.f : 1.f;
+    bool wrap = false;
+    for (int t = tid; t < 32 * m; t += kListThreads) {
+        const int J = nb.j[(size_t)I * nb.cap + (t >> 5)] * 32 + (t & 31);
+        const float4 x = a.xs[J], p = nb.ljs[J];
+        px[t] = make_float4(x.x, x.y, x.z, p.x);
+        if (SAME) le2[t] = make_float2(er_on * p.y, ea_on * p.z);
+        else le4[t] = make_float4(er_on * p.y, ea_on * p.z, p.w, 0.f);
     }
-    blk -= a.blocks_angles;
-    if (blk < a.blocks_dih) {
-        const int t = blk * kForceThreads + threadIdx.x;
-        float efld = 0.f, egd = 0.f;
-        if (t < a.n_dih) {
-            const DihedralTerm q = a.dih[t];
-            const int slot = q.kind == kDihFLD ? kSlotFLD : kSlotGD;
-            if (a.slots_enabled & (1u << slot)) {
-                const float3 F = bonded_sep(a, q.j, q.i, q.periodic);  // x1 - x2
-                const float3 G = bonded_sep(a, q.k, q.j, q.periodic);  // x2 - x3
-                const float3 H = bonded_sep(a, q.k, q.l, q.periodic);  // x4 - x3
-                float3 f1, f2, f3, f4;
-                float en;
-                const Torsion g = torsion_geometry(F, G, H);
-                if (q.kind == kDihFLD) {
-                    fld_forces(g, F, G, H, q.kk, a.fld[q.table], f1, f2, f3, f4, en);
-                    efld = en;
-                } else {
-                    gauss_dihedral_forces(g, F, G, H, q.kk, q.theta0, q.inv2s2, f1, f2, f3, f4, en);
-                    egd = en;
-                }
-                add_force(a, q.i, f1);
-                add_force(a, q.j, f2);
-                add_force(a, q.k, f3);
-                add_force(a, q.l, f4);
-            }
-        }
-        if (ENERGY) {
-            const double v = warp_sum((double)efld), vg = warp_sum((double)egd);
-            if (lane == 0) {
-                if (v != 0.0) atomicAdd(&a.energy[kSlotFLD], v);
-                if (vg != 0.0) atomicAdd(&a.energy[kSlotGD], vg);
-            }
-        }
-        return;
+    for (int t = tid; t < m; t += kListThreads) {
+        sA[t] = nb.shift[(size_t)I * nb.cap + t];
+        wrap = wrap || sA[t].w != 0.f;
     }
-    blk -= a.blocks_dih;
-    {
-        // ---------------- charged pairs (Debye-Hueckel) ----------------
-        // One warp per charged bead over its row; each pair's force on bead
-        // i is rounded to fixed point and summed as integers, then added
-        // once per bead.
-        const int warp = threadIdx.x >> 5;
-        float edh = 0.f;
-        if (a.slots_enabled & (1u << kSlotDH)) {
-            const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int t = blk * kWarpsPerForceBlock + warp; t < a.n_chg; t += a.blocks_chg * kWarpsPerForceBlock) {
-                const int i = a.chg_idx[t];
-                const float4 xi = a.xq[i], li = a.xlo[i];
-                const float4 pi = a.p0[i];
-                const int len = min(a.chg_len[t], a.chg_row_cap);
-                const int32_t* row = a.chg_rows + (size_t)t * a.chg_row_cap;
-                long long fx = 0, fy = 0, fz = 0;
-                bool bad = false;
-                for (int p = lane; p < len; p += 32) {
-                    const int j = row[p];
-                    const float3 d = ff_separation<PERIODIC>(xi, li, a.xq[j], a.xlo[j], a.box, a.inv_box);
-                    const float r2 = norm2(d);
-                    if (r2 < a.pc.dh_rc2) {
-                        PairEnergy e;
-                        e.zero();
-                        const float sc = pair_scalar<kTermDH, ENERGY>(r2, pi, a.p0[j], zero4, zero4, 0u, a.pc, e);
-                        bad = bad || !force_ok(make_float3(sc * d.x, sc * d.y, sc * d.z));
-                        fx += (long long)to_fixed(-sc * d.x);
-                        fy += (long long)to_fixed(-sc * d.y);
-                        fz += (long long)to_fixed(-sc * d.z);
-                        if (ENERGY && i < j) edh += e.dh;
-                    }
-                }
+    if (tid == 0) {
+        px[dummy] = make_float4(1e15f, 1e15f, 1e15f, 0.f);
+        sA[nb.cap] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (SAME) le2[dummy] = make_float2(0.f, 0.f);
+        else le4[dummy] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float4 xi = a.xs[k], pi = nb.ljs[k];
+    const float4 lei = make_float4(er_on * pi.y, ea_on * pi.z, pi.w, 0.f);
+    wrap = __syncthreads_or(wrap);
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    double er = 0.0, ea = 0.0;
+    for (int g = 0; g < groups; ++g) {
+        const uint2 next = g + 1 < groups ? list[(size_t)(g + 1) * kListThreads] : e;
+        uint32_t ent[4] = {e.x & 0xFFFFu, e.x >> 16, e.y & 0xFFFFu, e.y >> 16};
+        float4 xj[4], A[4], lej[4];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-                    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-                    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-                }
-                if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.flags, ListFlags::kBlownUp);
-                if (lane == 0) {
-                    if (fx) atomicAdd(&a.F[i], (unsigned long long)fx);
-                    if (fy) atomicAdd(&a.F[a.n + i], (unsigned long long)fy);
-                    if (fz) atomicAdd(&a.F[2 * a.n + i], (unsigned long long)fz);
-                }
+        for (int u = 0; u < 4; ++u) {
+            xj[u] = *reinterpret_cast<const float4*>(smem + 2 * ent[u]);
+            A[u] = sA[ent[u] >> 8];
+            if (SAME) {
+                const float2 l = *reinterpret_cast<const float2*>(sle + ent[u]);
+                lej[u] = make_float4(l.x, l.y, 0.f, 0.f);
+            } else {
+                lej[u] = *reinterpret_cast<const float4*>(sle + 2 * ent[u]);
             }
         }
+        float er4 = 0.f, ea4 = 0.f;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            float3 d = anchored_sep(xi, xj[u], make_float3(A[u].x, A[u].y, A[u].z));
+            if (wrap && A[u].w != 0.f) d = min_image(d, a.box, a.inv_box);
+            lj_pair<SAME, ENERGY>(d, pi.x, xj[u].w, lei, lej[u], a.pc, f, er4, ea4);
+        }
         if (ENERGY) {
-            const double v = warp_sum((double)edh);
-            if (lane == 0 && v != 0.0) atomicAdd(&a.energy[kSlotDH], v);
+            er += (double)er4;
+            ea += (double)ea4;
+        }
+        e = next;
+    }
+    // the units of a bead, in a fixed order
+#pragma unroll
+    for (int o = 1; o < kListUnits; o <<= 1) {
+        f.x += __shfl_xor_sync(kFull, f.x, o);
+        f.y += __shfl_xor_sync(kFull, f.y, o);
+        f.z += __shfl_xor_sync(kFull, f.z, o);
+    }
+    if (tid % kListUnits == 0) {
+        const int o = a.perm[k];
+        if (o >= 0) add_force(a, o, f);
+    }
+    if (ENERGY) {  // a pair is met from both of its beads
+        const double vr = warp_sum(0.5 * er), va = warp_sum(0.5 * ea);
+        if ((tid & 31) == 0) {
+            if (vr != 0.0) atomicAdd(&a.energy[kSlotLJR], vr);
+            if (va != 0.0) atomicAdd(&a.energy[kSlotLJA], va);
         }
     }
 }
@@ -1157,6 +1546,52 @@ __global__ void k_list_pairs(int nc, const float4* __restrict__ xs, const float4
     }
 }
 
+// The same verification for the pair lists: every listed pair (from its
+// lower bead) whose FP32 r^2 is below the cutoff squared ...
+__global__ void k_list_entries(int nc, const float4* __restrict__ xs, const int32_t* __restrict__ perm, NeighbourLists nb,
+                               float3 box, float3 inv_box, float rc2, long long* out, long long cap,
+                               unsigned long long* count) {
+    const int I = blockIdx.x, unit = threadIdx.x;
+    if (nb.cnt[I] == 0) return;
+    const int k = I * 32 + unit / kListUnits;
+    const int oi = perm[k];
+    const int mine = unit_entries(nb.len[k], unit % kListUnits);
+    for (int p = 0; p < mine; ++p) {
+        const int e = nb.list[list_at(nb, I, p, unit)] >> 3;
+        const size_t at = (size_t)I * nb.cap + (e >> 5);
+        const int kj = nb.j[at] * 32 + (e & 31), oj = perm[kj];
+        const float4 A = nb.shift[at];
+        float3 d = anchored_sep(xs[k], xs[kj], make_float3(A.x, A.y, A.z));
+        d = min_image(d, box, inv_box);
+        if (oi < oj && norm2(d) < rc2) {
+            const unsigned long long to = atomicAdd(count, 1ull);
+            if ((long long)to < cap) {
+                out[2 * to] = oi;
+                out[2 * to + 1] = oj;
+            }
+        }
+    }
+}
+// ... and the pairs that the lists leave out as excluded.
+__global__ void k_excluded_pairs(int nnz, const int32_t* __restrict__ ex_i, const int32_t* __restrict__ ex_j,
+                                 const uint8_t* __restrict__ ex_bits, const int32_t* __restrict__ slot,
+                                 const float4* __restrict__ xs, const float4* __restrict__ anc, BoxD bd, float3 box,
+                                 float3 inv_box, float rc2, long long* out, long long cap,
+                                 unsigned long long* count) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nnz || ex_i[e] >= ex_j[e] || !(ex_bits[e] & kTermLJR)) return;
+    const int ki = slot[ex_i[e]], kj = slot[ex_j[e]];
+    float3 d = anchored_sep(xs[ki], xs[kj], anchor_shift(anc[ki >> 5], anc[kj >> 5], bd));
+    d = min_image(d, box, inv_box);
+    if (norm2(d) < rc2) {
+        const unsigned long long to = atomicAdd(count, 1ull);
+        if ((long long)to < cap) {
+            out[2 * to] = ex_i[e];
+            out[2 * to + 1] = ex_j[e];
+        }
+    }
+}
+
 template <int TERMS>
 void launch_forces_t(const ForceArgs& a, int grid, cudaStream_t s, bool periodic, bool energy) {
     if (periodic) {
@@ -1308,6 +1743,24 @@ PlainContext::PlainContext(const SystemDesc& d, double temperature, double frict
                 chg_row_cap_ = 128;
                 chg_rows_.alloc(n_charged_ * chg_row_cap_);
             }
+        }
+    }
+    // Per-bead pair lists instead of tiles: both Lennard-Jones terms with
+    // arithmetic epsilons and the same excluded pairs, no interaction groups,
+    // the column layout, and Debye-Hueckel absent or on its charged rows.
+    {
+        const int tile_terms = cs.pc.terms & ~(charged_split_ ? kTermDH : 0);
+        bool same = true;
+        for (uint8_t b : cs.ex_bits) same = same && ((b & kTermLJR) != 0) == ((b & kTermLJA) != 0);
+        // (leave_pair_lists: a neighbourhood of more than kMaxNeighbours
+        // clusters or kMaxColumns columns does not fit a block)
+        pair_lists_ = reorder && tile_terms == (kTermLJR | kTermLJA) && same && !cs.pc.ljr_geometric &&
+                      !(cs.pc.uses_labels & (kTermLJR | kTermLJA));
+        if (pair_lists_) {
+            nbr_cap_ = 48;
+            list_cap_ = 24;
+            ljs_.alloc(np);
+            alloc_pair_lists();
         }
     }
     bonds_.upload(cs.bonds, s);
@@ -1486,7 +1939,7 @@ void PlainContext::rebuild(cudaStream_t s) {
     const BoxD bd = box_d();
     k_gather_sorted<<<div_up(np, 256), 256, 0, s>>>(np_i, perm_.p, xq_.p, x_.p, y_.p, z_.p, bd, p0_.p, p1_.p,
                                                     lab_.p, slot_.p, xs_.p, anc_.p, p0s_.p, p1s_.p, labs_.p,
-                                                    ref_.p);
+                                                    ref_.p, pair_lists_ ? ljs_.p : nullptr);
     const bool per = cs.periodic;
     const int wblocks = div_up(nc * 32, 128);
     k_bbox<<<wblocks, 128, 0, s>>>(nc_i, xs_.p, anc_.p, perm_.p, bb_c_.p, bb_h_.p);
@@ -1494,6 +1947,12 @@ void PlainContext::rebuild(cudaStream_t s) {
                                                ext_.p);
     const float cut = (float)(tile_cutoff_ + skin) * 1.0001f + 1e-4f;
     const float cut2 = cut * cut;
+    if (int reach[2]; pair_lists_ && column_reach(cut, reach) > kMaxColumns) leave_pair_lists();
+    if (pair_lists_) {
+        rebuild_pair_lists(s, cut);
+        rebuild_charged_rows(s);
+        return;
+    }
     if (per) {
         k_tiles<true, false><<<wblocks, 128, 0, s>>>(nc_i, bb_c_.p, bb_h_.p, box_, inv_box_, cut, cut2,
                                                      tile_count_.p, nullptr, nullptr, nullptr, 0, flags_.p);
@@ -1533,6 +1992,10 @@ void PlainContext::rebuild(cudaStream_t s) {
                                                        flags_.p);
     }
     OCM_CK(cudaGetLastError());
+    rebuild_charged_rows(s);
+}
+
+void PlainContext::rebuild_charged_rows(cudaStream_t s) {
     if (charged_split_) {
         // cell sort done with the beads' (the split implies the reordered layout)
         const int m = (int)n_charged_;
@@ -1542,6 +2005,70 @@ void PlainContext::rebuild(cudaStream_t s) {
             inv_box_, ccut * ccut, chg_start_.p, chg_sorted_.p, ex_csr_.p, ex_j_.p, ex_bits_.p, chg_rows_.p,
             chg_len_.p, (int)chg_row_cap_, chg_stats_.p, flags_.p);
     }
+}
+
+// Neighbour clusters and per-bead lists of the cluster order just built.
+void PlainContext::rebuild_pair_lists(cudaStream_t s, float cut) {
+    const NeighbourLists nb = neighbour_lists();
+    const int nc_i = (int)nc;
+    int reach[2];
+    column_reach(cut, reach);
+    OCM_CK(cudaMemsetAsync(nbr_stats_.p, 0, 3 * sizeof(int32_t), s));
+    k_pair_lists<<<nc_i, kBuildThreads, list_smem(false, true), s>>>(
+        nc_i, cell_dims_[0], cell_dims_[1], cell_dims_[2], reach[0], reach[1], perm_.p, cell_key_.p, col_start_.p, slot_.p,
+        xs_.p, bb_c_.p, bb_h_.p, ext_.p, box_d(), box_, inv_box_, wrap_pad(), cut, ex_csr_.p, ex_j_.p, ex_bits_.p, nb);
+    OCM_CK(cudaGetLastError());
+}
+
+// Columns to either side that can hold a neighbour (their gap stays below
+// the cutoff); returns how many columns a neighbourhood spans.
+int PlainContext::column_reach(float cut, int reach[2]) const {
+    int span = 1;
+    for (int a = 0; a < 2; ++a) {
+        reach[a] = (int)((cut + 1e-3) / (cs.box[a] / cell_dims_[a])) + 1;
+        span *= std::min(cell_dims_[a], 2 * reach[a] + 1);
+    }
+    return span;
+}
+
+NeighbourLists PlainContext::neighbour_lists() const {
+    NeighbourLists nb{};
+    nb.cap = nbr_cap_;
+    nb.list_groups = list_cap_ / 4;
+    nb.cnt = nbr_cnt_.p;
+    nb.j = nbr_j_.p;
+    nb.shift = nbr_shift_.p;
+    nb.len = list_len_.p;
+    nb.list = list_.p;
+    nb.ljs = ljs_.p;
+    nb.stats = nbr_stats_.p;
+    nb.flags = flags_.p;
+    return nb;
+}
+
+// Shared memory of a pair-list block: staged positions and shifts, and for
+// the force kernel the Lennard-Jones parameters.
+size_t PlainContext::list_smem(bool same_sigma, bool build) const {
+    const size_t beads = 32 * (size_t)nbr_cap_ + 1;
+    return 16 * beads + 16 * ((size_t)nbr_cap_ + 1) + (build ? 0 : (same_sigma ? 8 : 16) * beads);
+}
+
+void PlainContext::alloc_pair_lists() {
+    nbr_cnt_.alloc(nc);
+    nbr_j_.alloc(nc * nbr_cap_);
+    nbr_shift_.alloc(nc * nbr_cap_);
+    list_len_.alloc(nc * 32);
+    list_.alloc(nc * (size_t)kListThreads * list_cap_);
+    nbr_stats_.alloc(3);
+    // an evaluation before the first build finds empty lists
+    OCM_CK(cudaMemsetAsync(nbr_cnt_.p, 0, nc * sizeof(int32_t), stream_));
+    OCM_CK(cudaMemsetAsync(list_len_.p, 0, nc * 32 * sizeof(int32_t), stream_));
+    // the limit is the kernels', not this context's: always the largest
+    const int most = 32 * kMaxNeighbours + 1, bytes = 32 * most + 16 * (kMaxNeighbours + 1);
+    const void* fns[] = {(const void*)k_forces_lists<true, false>,  (const void*)k_forces_lists<true, true>,
+                         (const void*)k_forces_lists<false, false>, (const void*)k_forces_lists<false, true>,
+                         (const void*)k_pair_lists};
+    for (const void* f : fns) OCM_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
 void PlainContext::launch_forces(cudaStream_t s, bool energy, uint32_t slots_enabled, int) {
@@ -1556,9 +2083,10 @@ void PlainContext::launch_forces(cudaStream_t s, bool energy, uint32_t slots_ena
     a.n_bonds = (int)cs.bonds.size();
     a.n_angles = (int)cs.angles.size();
     a.n_dih = (int)cs.dihedrals.size();
-    a.blocks_bonds = div_up(a.n_bonds, kForceThreads);
-    a.blocks_angles = div_up(a.n_angles, kForceThreads);
-    a.blocks_dih = div_up(a.n_dih, kForceThreads);
+    const int threads = pair_lists_ ? kListThreads : kForceThreads;
+    a.blocks_bonds = div_up(a.n_bonds, threads);
+    a.blocks_angles = div_up(a.n_angles, threads);
+    a.blocks_dih = div_up(a.n_dih, threads);
     a.xs = xs_.p; a.p0s = p0s_.p; a.p1s = p1s_.p; a.labs = labs_.p; a.perm = perm_.p;
     a.tile_start = tile_start_.p; a.tile_i = tile_i_.p; a.tile_j = tile_j_.p; a.tile_mask = tile_mask_.p;
     a.masks = masks_.p;
@@ -1589,8 +2117,12 @@ void PlainContext::launch_forces(cudaStream_t s, bool energy, uint32_t slots_ena
     a.n_chg = (int)n_charged_;
     a.chg_row_cap = (int)chg_row_cap_;
     a.flags = flags_.p;
-    a.blocks_chg = charged_split_ ? (int)std::max<int64_t>(1, div_up(n_charged_, kWarpsPerForceBlock)) : 0;
+    a.blocks_chg = charged_split_ ? (int)std::max<int64_t>(1, div_up(n_charged_, threads / 32)) : 0;
     a.energy = energy_.p;
+    if (pair_lists_) {
+        a.nb = neighbour_lists();
+        a.blocks_tiles = (int)nc;
+    }
     int blocks_tiles = a.blocks_tiles;
     if ((cs.pc.terms & ~excl_all & 15) == 0) {
         a.blocks_tiles = 0;
@@ -1601,7 +2133,14 @@ void PlainContext::launch_forces(cudaStream_t s, bool energy, uint32_t slots_ena
     // the tiles' pair terms (Debye-Hueckel leaves them for the charged rows)
     const int terms = cs.pc.terms & ~(charged_split_ ? kTermDH : 0);
     const bool per = cs.periodic;
-    if ((terms & ~(kTermEXV | kTermDH)) == 0) launch_forces_t<kTermEXV | kTermDH>(a, grid, s, per, energy);
+    if (pair_lists_) {
+        const bool same = cs.lj_same_sigma && cs.pc.ljr_rc2 == cs.pc.lja_rc2;
+        const size_t smem = list_smem(same, false);
+        if (same && energy) k_forces_lists<true, true><<<grid, kListThreads, smem, s>>>(a);
+        else if (same) k_forces_lists<true, false><<<grid, kListThreads, smem, s>>>(a);
+        else if (energy) k_forces_lists<false, true><<<grid, kListThreads, smem, s>>>(a);
+        else k_forces_lists<false, false><<<grid, kListThreads, smem, s>>>(a);
+    } else if ((terms & ~(kTermEXV | kTermDH)) == 0) launch_forces_t<kTermEXV | kTermDH>(a, grid, s, per, energy);
     else if (terms == (kTermLJR | kTermLJA) && cs.lj_same_sigma)
         launch_forces_t<kTermLJR | kTermLJA | kLJSameSigma>(a, grid, s, per, energy);
     else if ((terms & ~(kTermLJR | kTermLJA)) == 0) launch_forces_t<kTermLJR | kTermLJA>(a, grid, s, per, energy);
@@ -1641,19 +2180,40 @@ void PlainContext::ensure_capacity() {
     for (int attempt = 0; attempt < 8; ++attempt) {
         OCM_CK(cudaMemsetAsync(flags_.p, 0, sizeof(int32_t), stream_));
         rebuild(stream_);
-        int32_t total = 0, masks = 0, flags = 0, chg[2] = {0, 0};
+        int32_t total = 0, masks = 0, flags = 0, chg[2] = {0, 0}, nbr[3] = {0, 0, 0};
         if (charged_split_)
             OCM_CK(cudaMemcpyAsync(chg, chg_stats_.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
         int32_t kept = 0;  // tiles after pruning
-        OCM_CK(cudaMemcpyAsync(&total, raw_start_.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
-        OCM_CK(cudaMemcpyAsync(&kept, tile_start_.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
-        OCM_CK(cudaMemcpyAsync(&masks, mask_count_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+        if (pair_lists_) {
+            OCM_CK(cudaMemcpyAsync(nbr, nbr_stats_.p, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+        } else {
+            OCM_CK(cudaMemcpyAsync(&total, raw_start_.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+            OCM_CK(cudaMemcpyAsync(&kept, tile_start_.p + nc, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+            OCM_CK(cudaMemcpyAsync(&masks, mask_count_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+        }
         OCM_CK(cudaMemcpyAsync(&flags, flags_.p, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
         OCM_CK(cudaStreamSynchronize(stream_));
         // A buffer that is reallocated loses the list just built into it, so
         // any growth (also the pre-emptive one below 80% headroom) is
         // followed by another build before the list is used.
         bool realloced = false;
+        if (pair_lists_) {
+            if (nbr[0] > kMaxNeighbours) {  // more neighbours than a block can stage: the tiles from here on
+                leave_pair_lists();
+                continue;
+            }
+            // a few neighbours and 20% of list entries to spare
+            const int want_n = std::min(kMaxNeighbours, (nbr[0] + 3) / 4 * 4 + 4);
+            const int want_l = (nbr[1] * 3 / 2 + 4 + 3) / 4 * 4;
+            if (nbr[0] > nbr_cap_ || (nbr[0] + 2 > nbr_cap_ && nbr_cap_ < want_n) || nbr[1] * 6 / 5 + 2 > list_cap_) {
+                nbr_cap_ = std::max(nbr_cap_, want_n);
+                list_cap_ = std::max(list_cap_, want_l);
+                alloc_pair_lists();
+                realloced = true;
+                clear_graphs();
+            }
+            kept = nbr[2];
+        }
         if (total > tile_cap_ || (int64_t)total * 5 / 4 + 64 > tile_cap_) {
             const int64_t want = std::min<int64_t>(nc * (nc + 1) / 2, (int64_t)total * 2 + 1024);
             if (want > tile_cap_) {
@@ -1683,7 +2243,8 @@ void PlainContext::ensure_capacity() {
             }
         }
         if (!realloced &&
-            !(flags & (ListFlags::kTileOverflow | ListFlags::kMaskOverflow | ListFlags::kChargedOverflow)) &&
+            !(flags & (ListFlags::kTileOverflow | ListFlags::kMaskOverflow | ListFlags::kChargedOverflow |
+                       ListFlags::kListOverflow | ListFlags::kNeighbourOverflow)) &&
             total <= tile_cap_ && masks <= mask_cap_ && chg[0] <= chg_row_cap_) {
             tiles_last = kept;
             masked_last = masks;
@@ -1913,6 +2474,15 @@ void PlainContext::step(int64_t nsteps) {
             chg_row_cap_ *= 2;
             chg_rows_.alloc(n_charged_ * chg_row_cap_);
         }
+        if (flags & (ListFlags::kListOverflow | ListFlags::kNeighbourOverflow)) {
+            if ((flags & ListFlags::kNeighbourOverflow) && nbr_cap_ == kMaxNeighbours) {
+                leave_pair_lists();
+            } else {
+                if (flags & ListFlags::kNeighbourOverflow) nbr_cap_ = std::min(kMaxNeighbours, nbr_cap_ + 8);
+                else list_cap_ += 4 + list_cap_ / 16 * 4;
+                alloc_pair_lists();
+            }
+        }
         if (flags & (ListFlags::kTileOverflow | ListFlags::kMaskOverflow)) {
             tile_cap_ = std::min<int64_t>(nc * (nc + 1) / 2, tile_cap_ * 2);
             alloc_tile_arrays();
@@ -1923,6 +2493,12 @@ void PlainContext::step(int64_t nsteps) {
         ensure_capacity();
     }
     throw Error(4, "[error] step could not complete after repeated list rebuilds");
+}
+
+// Back to the tiles, for a system whose neighbourhoods do not fit a block.
+void PlainContext::leave_pair_lists() {
+    pair_lists_ = false;
+    clear_graphs();
 }
 
 void PlainContext::set_list_options(int32_t interval, double sk) {
@@ -2009,7 +2585,16 @@ void PlainContext::list_pairs(int64_t* out, int64_t cap, int64_t* n_out) {
     OCM_CK(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long), stream_));
     const int wblocks = div_up(nc * 32, 128);
     const float tile_rc2 = charged_split_ ? (float)(tile_cutoff_ * tile_cutoff_) : cs.pc.list_rc2;
-    if (cs.periodic)
+    if (pair_lists_) {
+        const NeighbourLists nb = neighbour_lists();
+        k_list_entries<<<(int)nc, kListThreads, 0, stream_>>>((int)nc, xs_.p, perm_.p, nb, box_, inv_box_, tile_rc2, buf.p,
+                                                               cap, cnt.p);
+        const int nnz = (int)cs.ex_j.size();
+        if (nnz > 0)
+            k_excluded_pairs<<<div_up(nnz, 256), 256, 0, stream_>>>(nnz, ex_start_.p, ex_j_.p, ex_bits_.p, slot_.p, xs_.p,
+                                                                    anc_.p, box_d(), box_, inv_box_, tile_rc2, buf.p, cap,
+                                                                    cnt.p);
+    } else if (cs.periodic)
         k_list_pairs<true><<<wblocks, 128, 0, stream_>>>((int)nc, xs_.p, tile_shift_.p, perm_.p, tile_start_.p,
                                                         tile_j_.p, box_, inv_box_, tile_rc2,
                                                         buf.p, cap, cnt.p, tile_cap_);

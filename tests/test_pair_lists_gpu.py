@@ -1,0 +1,68 @@
+"""The per-bead pair lists of the plain path (both Lennard-Jones terms of a
+large periodic system) where they can go wrong: against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from conftest import rel_force_err
+
+pytestmark = pytest.mark.gpu
+
+FORCE_TOL = 1e-4   # FP32 pair arithmetic, the bar of the parity tests
+ENERGY_TOL = 1e-5
+
+
+def _slab(kind):
+    from opencafemol_gb300 import synth
+    if kind == "narrow":  # 6 nm wide: neighbour shifts near half the box need the minimum image
+        spec = synth.hps_slab(23, 97, (6.0, 6.5, 110.0), slab_width=40.0, seed=3, dh_cutoff=2.2)
+        spec.dh = None
+        return spec
+    cutoff = {"far": 4.0}.get(kind, 2.0)  # 4 nm: more neighbour clusters than a block stages, so tiles
+    spec = synth.hps_slab(23, 97, (15.0, 15.0, 50.0), slab_width=14.0, seed=5, hps_cutoff=cutoff)
+    if kind == "sigmas":  # the two terms' sigmas differ, and with them the cutoffs
+        spec.lja.p1 = spec.lja.p1 * np.random.default_rng(1).uniform(0.9, 1.1, spec.n)
+    elif kind == "molecules":  # exclusion rows of 96 partners
+        spec.ljr.ign_molecule = spec.lja.ign_molecule = True
+    elif kind == "empty":  # no attraction: zero epsilons
+        spec.lja.p0 = np.zeros(spec.n)
+    return spec
+
+
+@pytest.mark.parametrize("kind", ["plain", "sigmas", "molecules", "empty", "narrow", "far"])
+def test_forces_and_energies(gpu, kind):
+    from opencafemol_gb300 import synth
+    from oracle import oracle
+    spec = _slab(kind)
+    system = synth.build_system(spec)
+    ctx = gpu.Context(system, gpu.LangevinIntegrator(spec.temperature, 5.0, 0.002, 7))
+    ctx.setPositions(spec.pos)
+    ctx.setVelocitiesToTemperature(spec.temperature, 3)
+    L = np.asarray(spec.box)
+    for _ in range(2):  # as packed, and after the lists were rebuilt during a run
+        f, _ = ctx.getState(energy=False)
+        x = ctx.getPositions()
+        f_ref, e_ref = oracle.evaluate(spec, pos=x)
+        assert rel_force_err(f, f_ref) <= FORCE_TOL
+        e = ctx.getGroupEnergies()
+        for g, name in enumerate(system.group_names()):
+            assert abs(e[g] - e_ref[name]) <= ENERGY_TOL * max(1.0, abs(e_ref[name])), name
+        ctx.step(200)
+        x = ctx.getPositions()
+        x = (x - L * np.floor(x / L)).astype(np.float32).astype(np.float64)
+        ctx.setPositions(np.where(x >= L, x - L, x))  # FP32-exact for both sides
+    assert ctx.stats()["reordered"] == 1
+
+
+def test_repeated_runs_are_bit_identical(gpu):
+    """List order and sums do not depend on the timing of the build."""
+    from opencafemol_gb300 import synth
+    spec = _slab("plain")
+    system = synth.build_system(spec)
+    out = []
+    for _ in range(2):
+        ctx = gpu.Context(system, gpu.LangevinIntegrator(spec.temperature, 5.0, 0.002, 7))
+        ctx.setPositions(spec.pos)
+        ctx.setVelocitiesToTemperature(spec.temperature, 3)
+        ctx.step(120)
+        out.append((ctx.getPositions(), ctx.getVelocities()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])

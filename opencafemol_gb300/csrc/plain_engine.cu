@@ -112,14 +112,23 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Exclusive scan of m ints into out[0..m] (out[m] = total) by one block of
 // 1024 threads: each of the 32 warps owns a contiguous segment and reads it
 // 32 consecutive values at a time (coalesced) - once for the segment total,
-// once more to write the prefixes with a shuffle scan.
+// once more to write the prefixes with a shuffle scan.  One block is all
+// latency, so kScanUnroll such rows are in flight at once (16 -> 13 us on
+// average over slabs of 3,007 to 200,000 beads).
+constexpr int kScanUnroll = 8;
 __device__ __forceinline__ void block_scan(int m, const int32_t* __restrict__ in, int32_t* __restrict__ out) {
     __shared__ int32_t wsum[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int per = (m + 31) / 32;
     const int b = w * per, e = min(m, b + per);
     int32_t s = 0;
-    for (int i = b + lane; i < e; i += 32) s += in[i];
+    for (int i = b + lane; i < e; i += 32 * kScanUnroll) {
+        int32_t v[kScanUnroll];
+#pragma unroll
+        for (int u = 0; u < kScanUnroll; ++u) v[u] = i + 32 * u < e ? in[i + 32 * u] : 0;
+#pragma unroll
+        for (int u = 0; u < kScanUnroll; ++u) s += v[u];
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
     if (lane == 0) wsum[w] = s;
@@ -135,17 +144,23 @@ __device__ __forceinline__ void block_scan(int m, const int32_t* __restrict__ in
     }
     __syncthreads();
     int32_t run = w > 0 ? wsum[w - 1] : 0;
-    for (int i0 = b; i0 < e; i0 += 32) {  // warp-uniform bounds
-        const int i = i0 + lane;
-        const int32_t v = i < e ? in[i] : 0;
-        int32_t x = v;
+    for (int i0 = b; i0 < e; i0 += 32 * kScanUnroll) {  // warp-uniform bounds
+        int32_t v[kScanUnroll], x[kScanUnroll];
+#pragma unroll
+        for (int u = 0; u < kScanUnroll; ++u) x[u] = v[u] = i0 + 32 * u + lane < e ? in[i0 + 32 * u + lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int32_t u = __shfl_up_sync(kFull, x, o);
-            if (lane >= o) x += u;
+#pragma unroll
+            for (int u = 0; u < kScanUnroll; ++u) {
+                const int32_t y = __shfl_up_sync(kFull, x[u], o);
+                if (lane >= o) x[u] += y;
+            }
         }
-        if (i < e) out[i] = run + x - v;
-        run += __shfl_sync(kFull, x, 31);
+#pragma unroll
+        for (int u = 0; u < kScanUnroll; ++u) {
+            if (i0 + 32 * u + lane < e) out[i0 + 32 * u + lane] = run + x[u] - v[u];
+            run += __shfl_sync(kFull, x[u], 31);
+        }
     }
     if (threadIdx.x == 0) out[m] = wsum[31];
 }
@@ -566,10 +581,13 @@ __global__ void k_scatter_both(int n, const int32_t* __restrict__ key, const int
     }
 }
 
-// One warp per charged bead: the 27 neighbour cells (the three cells of a
-// row along x as one range where they do not wrap), 32 candidates at a time,
-// kept partners compacted by ballot.  row_stats[0] is the longest row,
-// row_stats[1] the number of row entries.
+// One warp per charged bead: the candidates of the 27 neighbour cells, 32 at
+// a time, kept partners compacted by ballot.  Latency-bound: the ranges of
+// the cells are read at once and kRowUnroll rows of candidates are in flight,
+// where a loop over ranges waited for each in turn.  Per launch: 600 charged
+// beads 20 -> 8 us, 4,000 32 -> 23, 40,000 147 -> 125.
+// row_stats[0] is the longest row, row_stats[1] the number of row entries.
+constexpr int kRowUnroll = 4;
 __global__ void k_chg_rows(int m, const int32_t* __restrict__ idx, const int32_t* __restrict__ key,
                            const float4* __restrict__ xq, int nx, int ny, int nz, float3 box,
                            float3 inv_box, float cut2, const int32_t* __restrict__ start,
@@ -589,44 +607,63 @@ __global__ void k_chg_rows(int m, const int32_t* __restrict__ idx, const int32_t
     // outside skip the search
     const int ex_lo = e0 < e1 ? ex_j[e0] : 1, ex_hi = e0 < e1 ? ex_j[e1 - 1] : 0;
     int32_t* row = rows + (size_t)t * row_cap;
+    // The neighbour cells as ranges of `sorted`, one per lane (three along x
+    // are one range where they do not wrap), and their candidates as one
+    // sequence: lane l's range starts at base there.
+    const bool inner = cx > 0 && cx < nx - 1;
+    const int ranges = inner ? 9 : 27;
+    int q_begin = 0, q_count = 0;
+    if (lane < ranges) {
+        const int zy = inner ? lane : lane / 3;
+        const int r = (((cz + zy / 3 - 1 + nz) % nz) * ny + (cy + zy % 3 - 1 + ny) % ny) * nx;
+        const int c = inner ? cx - 1 : (cx + lane % 3 - 1 + nx) % nx;
+        q_begin = start[r + c];
+        q_count = start[r + c + (inner ? 3 : 1)] - q_begin;
+    }
+    int incl = q_count;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, s);
+        if (lane >= s) incl += u;
+    }
+    const int base = incl - q_count, total = __shfl_sync(0xffffffffu, incl, 31);
     int len = 0;
-    for (int dz = -1; dz <= 1; ++dz)
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int r = (((cz + dz + nz) % nz) * ny + (cy + dy + ny) % ny) * nx;
-            const bool inner = cx > 0 && cx < nx - 1;
-            for (int seg = 0; seg < (inner ? 1 : 3); ++seg) {
-                const int q_begin = inner ? start[r + cx - 1] : start[r + (cx + seg - 1 + nx) % nx];
-                const int q_end = inner ? start[r + cx + 2] : start[r + (cx + seg - 1 + nx) % nx + 1];
-                for (int q0 = q_begin; q0 < q_end; q0 += 32) {
-                    const int q = q0 + lane;
-                    bool keep = false;
-                    int j = 0;
-                    if (q < q_end) {
-                        const float4 c = sorted[q];
-                        j = __float_as_int(c.w);
-                        if (j != i) {
-                            const float r2 = norm2(separation<true>(xi, c, box, inv_box));
-                            keep = r2 < cut2;
-                            if (keep && j >= ex_lo && j <= ex_hi) {
-                                int lo = e0, hi = e1;  // this row's exclusions, sorted by j
-                                while (lo < hi) {
-                                    const int mid = (lo + hi) >> 1;
-                                    if (ex_j[mid] < j) lo = mid + 1;
-                                    else hi = mid;
-                                }
-                                if (lo < e1 && ex_j[lo] == j && (ex_bits[lo] & kTermDH)) keep = false;
-                            }
-                        }
-                    }
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const int at = len + __popc(bal & ((1u << lane) - 1u));
-                        if (at < row_cap) row[at] = j;
-                    }
-                    len += __popc(bal);
-                }
+    for (int p0 = 0; p0 < total; p0 += 32 * kRowUnroll) {
+        float4 c[kRowUnroll];
+#pragma unroll
+        for (int u = 0; u < kRowUnroll; ++u) {
+            const int p = p0 + 32 * u + lane;
+            // the last range that starts at or before p (binary search over lanes)
+            int at = 0;
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) {
+                const int v = __shfl_sync(0xffffffffu, base, at + s);
+                if (v <= p) at += s;
             }
+            const int q = __shfl_sync(0xffffffffu, q_begin, at) + p - __shfl_sync(0xffffffffu, base, at);
+            c[u] = p < total ? sorted[q] : make_float4(0.f, 0.f, 0.f, __int_as_float(i));
         }
+#pragma unroll
+        for (int u = 0; u < kRowUnroll; ++u) {
+            const int j = __float_as_int(c[u].w);
+            bool keep = j != i && norm2(separation<true>(xi, c[u], box, inv_box)) < cut2;
+            if (keep && j >= ex_lo && j <= ex_hi) {
+                int lo = e0, hi = e1;  // this row's exclusions, sorted by j
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (ex_j[mid] < j) lo = mid + 1;
+                    else hi = mid;
+                }
+                if (lo < e1 && ex_j[lo] == j && (ex_bits[lo] & kTermDH)) keep = false;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int at = len + __popc(bal & ((1u << lane) - 1u));
+                if (at < row_cap) row[at] = j;
+            }
+            len += __popc(bal);
+        }
+    }
     if (lane == 0) {
         row_len[t] = len;
         atomicMax(&row_stats[0], len);
@@ -669,10 +706,17 @@ __global__ void k_chg_list_pairs(int m, const int32_t* __restrict__ idx, const i
 // partners (adjacent lanes share a bead); a unit's entries are 8 x the staged
 // slot, in groups of four, the groups of a cluster's units side by side; the
 // last group is filled up with the dummy bead behind the staged ones.
+//
+// Only 8% of a tile's pair slots lie within the cutoff and a 32-slot step
+// costs ~92 instructions whether one lane hits or all do; a list entry costs
+// about 65 and 70% of the entries are within the cutoff, so a step of the
+// 20,000-bead slab takes 14M warp instructions instead of 38M although every
+// pair is met twice.  Eight lanes per bead and 64 registers: with four lanes
+// and 80 registers the shared memory left 16 warps per SM, 29 us instead of
+// 22 per launch.  The tiles take 44.
 // ---------------------------------------------------------------------------
 constexpr int kMaxNeighbours = 128;  // so that an entry fits 16 bits
 constexpr int kMaxColumns = 512;     // columns a neighbourhood may span
-constexpr int kMaxCandidates = 512;  // clusters whose boxes are in reach
 constexpr int kListUnits = 8;
 constexpr int kListThreads = 32 * kListUnits;
 constexpr int kBuildThreads = 512;
@@ -681,23 +725,37 @@ constexpr int kBuildWarps = kBuildThreads / 32;
 __device__ __forceinline__ size_t list_at(const NeighbourLists& nb, int I, int k, int unit) {
     return (((size_t)I * nb.list_groups + (k >> 2)) * kListThreads + unit) * 4 + (k & 3);
 }
+// Shared memory of the build's staged positions and, later, its rows.
+__host__ __device__ __forceinline__ int build_region(int cap, int list_groups) {
+    const int positions = 16 * 32 * cap, rows = 2 * kBuildWarps * kListUnits * 4 * list_groups;
+    return positions > rows ? positions : rows;
+}
 // Entries of unit s of a bead with len partners.
 __device__ __forceinline__ int unit_entries(int len, int s) { return (len - s + kListUnits - 1) / kListUnits; }
 
 // Neighbour clusters and lists of every cluster, one block each.
-//  1. The clusters of the columns within reach whose bounding boxes are
-//     within the cutoff (one warp per column: a count pass, then the same
-//     again to write them in column order).
-//  2. Of these, the ones where some bead of either is within the cutoff of
-//     the other's box (one warp each), in order, with their anchor shift and
-//     whether their pairs need the minimum image (see k_compact_tiles).
-//  3. One warp per bead: the lanes test the neighbour boxes, then 32 staged
-//     beads of each box that is near; hits are compacted by ballot.  A list
-//     holds the partners within cut (the canonical separation of the force
-//     kernel) that the exclusions keep, in neighbour order.
+//  1. Each warp looks through its share of the columns within reach: the
+//     clusters whose bounding boxes are within the cutoff and where some bead
+//     of either is within the cutoff of the other's box go to the warp's
+//     segment.
+//  2. The segments are joined in warp order; every neighbour gets its anchor
+//     shift and whether its pairs need the minimum image (see
+//     k_compact_tiles).
+//  3. Half a neighbour cluster per warp step, lane = bead of this cluster:
+//     16 staged beads tested one after another into a mask per lane.
+//  4. The excluded partners' bits are cleared, one thread per exclusion.
+//  5. One warp per bead: the lanes put the set bits of one mask after
+//     another in a row in shared memory (a lane per mask instead waits for
+//     the fullest, the cluster's own), which goes out in the units' order.
+//     A list holds the partners within cut (the canonical
+//     separation of the force kernel) that the exclusions keep, in
+//     neighbour order.
 // Columns within reach, not all clusters, and the two bead tests take the
 // place of the tiles' sweep over every cluster, exact pruning and exclusion
-// masks (eight launches).
+// masks (eight launches).  Issue-bound in 3 and 4: testing 32 beads of a
+// neighbour against one bead per warp step and compacting by ballot took
+// twice the instructions.  Per launch: 3,007 beads 24 -> 18 us, 20,000 beads
+// 71 -> 55, 200,000 beads 576 -> 450.
 __global__ void __launch_bounds__(kBuildThreads, 2)
     k_pair_lists(int nc, int nx, int ny, int nz, int rx, int ry, const int32_t* __restrict__ perm,
                  const int32_t* __restrict__ key, const int32_t* __restrict__ col_start,
@@ -707,171 +765,156 @@ __global__ void __launch_bounds__(kBuildThreads, 2)
                  const uint8_t* __restrict__ ex_bits, NeighbourLists nb) {
     extern __shared__ __align__(16) unsigned char smem[];
     float4* px = reinterpret_cast<float4*>(smem);
-    float4* sA = px + 32 * nb.cap + 1;
-    __shared__ int s_col[kMaxColumns + 1];
-    __shared__ int s_cand[kMaxCandidates];
-    __shared__ unsigned char s_keep[kMaxCandidates];
+    float4* sA = reinterpret_cast<float4*>(smem + build_region(nb.cap, nb.list_groups));
+    uint32_t* masks = reinterpret_cast<uint32_t*>(sA + nb.cap + 1);  // [neighbour][bead]
+    uint16_t* rows = reinterpret_cast<uint16_t*>(px);                 // a row per warp, once the positions are read
+    __shared__ int s_seg[kBuildWarps][kMaxNeighbours];
+    __shared__ int s_cnt[kBuildWarps];
     __shared__ int sj[kMaxNeighbours];
-    __shared__ int s_m;
     const int I = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float4 hi = bh[I];
     if (hi.w < 0.f) {  // padding slots only
         if (tid == 0) nb.cnt[I] = 0;
         return;
     }
+    // the exclusion rows of the cluster's beads (lane), one warp per entry
+    const int eb = perm[I * 32 + (tid & 31)], e0 = eb >= 0 ? ex_csr[eb] : 0, e1 = eb >= 0 ? ex_csr[eb + 1] : 0;
+    auto excluded_slot = [&](int e) { return e < e1 && (ex_bits[e] & kTermLJR) ? slot[ex_j[e]] : -1; };
+    const int first = excluded_slot(e0 + warp);
     const float cut2 = cut * cut;
     const float4 ci = bc[I];
     const int col = key[perm[I * 32]] / nz, cx = col % nx, cy = col / nx;
     const bool all_x = 2 * rx + 1 >= nx, all_y = 2 * ry + 1 >= ny;
     const int wx = all_x ? nx : 2 * rx + 1, columns = wx * (all_y ? ny : 2 * ry + 1);
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int v = warp; v < columns; v += kBuildWarps) {
-            const int ix = v % wx, iy = v / wx;
-            const int x = all_x ? ix : (cx - rx + ix + nx) % nx, y = all_y ? iy : (cy - ry + iy + ny) % ny;
-            const int q0 = col_start[y * nx + x] >> 5, q1 = col_start[y * nx + x + 1] >> 5;
-            int at = pass ? s_col[v] : 0;
-            for (int J = q0 + lane; J - lane < q1; J += 32) {
-                bool ok = false;
-                if (J < q1) {
-                    const float4 hj = bh[J];
-                    ok = hj.w >= 0.f && boxes_close<true>(ci, hi, bc[J], hj, box, inv_box, cut, cut2);
-                }
-                const unsigned bal = __ballot_sync(kFull, ok);
-                const int to = at + __popc(bal & ((1u << lane) - 1u));
-                if (pass && ok && to < kMaxCandidates) s_cand[to] = J;
-                at += __popc(bal);
-            }
-            if (!pass && lane == 0) s_col[v] = at;
-        }
-        __syncthreads();
-        if (!pass) {
-            if (warp == 0) {  // exclusive scan of the columns' counts
-                int run = 0;
-                for (int v0 = 0; v0 < columns; v0 += 32) {
-                    const int c = v0 + lane < columns ? s_col[v0 + lane] : 0;
-                    int incl = c;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int u = __shfl_up_sync(kFull, incl, o);
-                        if (lane >= o) incl += u;
-                    }
-                    if (v0 + lane < columns) s_col[v0 + lane] = run + incl - c;
-                    run += __shfl_sync(kFull, incl, 31);
-                }
-                if (lane == 0) s_col[columns] = run;
-            }
-            __syncthreads();
-        }
-    }
-    const int cands = min(s_col[columns], kMaxCandidates);
+    int found = 0, upper = 0;
     {
         const float4 xi = xs[I * 32 + lane];
-        for (int c = warp; c < cands; c += kBuildWarps) {
-            const int J = s_cand[c];
-            const float4 cj = bc[J], hj = bh[J], xj = xs[J * 32 + lane];
-            const float3 d = min_image(make_float3(cj.x - ci.x, cj.y - ci.y, cj.z - ci.z), box, inv_box);
-            auto near = [&](float4 x, float sign, float4 h) {  // false for padding (NaN)
-                const float gx = fmaxf(0.f, fabsf(d.x + sign * x.x) - h.x);
-                const float gy = fmaxf(0.f, fabsf(d.y + sign * x.y) - h.y);
-                const float gz = fmaxf(0.f, fabsf(d.z + sign * x.z) - h.z);
-                return x.x == x.x && gx * gx + gy * gy + gz * gz < cut2;
-            };
-            const bool wide = hi.x + hj.x + cut >= 0.5f * box.x || hi.y + hj.y + cut >= 0.5f * box.y ||
-                              hi.z + hj.z + cut >= 0.5f * box.z;
-            const bool keep = wide || (__any_sync(kFull, near(xi, -1.f, hj)) && __any_sync(kFull, near(xj, 1.f, hi)));
-            if (lane == 0) s_keep[c] = keep;
-        }
-    }
-    __syncthreads();
-    if (warp == 0) {
-        int m = 0, upper = 0;
-        const float4 ei = ext[I];
-        for (int c0 = 0; c0 < cands; c0 += 32) {
-            const bool keep = c0 + lane < cands && s_keep[c0 + lane];
-            const unsigned bal = __ballot_sync(kFull, keep);
-            const int to = m + __popc(bal & ((1u << lane) - 1u));
-            const int J = keep ? s_cand[c0 + lane] : I;
-            if (keep && to < nb.cap) {
-                const float3 A = anchor_shift(ci, bc[J], bd);
-                const float4 ej = ext[J];
-                const bool wrap = fabsf(A.x) + ei.x + ej.x + pad >= 0.5f * box.x ||
-                                  fabsf(A.y) + ei.y + ej.y + pad >= 0.5f * box.y ||
-                                  fabsf(A.z) + ei.z + ej.z + pad >= 0.5f * box.z;
-                const float4 shift = make_float4(A.x, A.y, A.z, wrap ? 1.f : 0.f);
-                sj[to] = J;
-                sA[to] = shift;
-                nb.j[(size_t)I * nb.cap + to] = J;
-                nb.shift[(size_t)I * nb.cap + to] = shift;
+        const int per = (columns + kBuildWarps - 1) / kBuildWarps, v0 = min(columns, warp * per),
+                  v1 = min(columns, v0 + per);
+        // the column ranges of up to 32 columns at once
+        for (int vb = v0; vb < v1; vb += 32) {
+            int q0 = 0, q1 = 0;
+            if (vb + lane < v1) {
+                const int ix = (vb + lane) % wx, iy = (vb + lane) / wx;
+                const int x = all_x ? ix : (cx - rx + ix + nx) % nx, y = all_y ? iy : (cy - ry + iy + ny) % ny;
+                q0 = col_start[y * nx + x] >> 5;
+                q1 = col_start[y * nx + x + 1] >> 5;
             }
-            upper += __popc(__ballot_sync(kFull, keep && J >= I));
-            m += __popc(bal);
+            for (int v = vb; v < min(v1, vb + 32); ++v) {
+                const int a0 = __shfl_sync(kFull, q0, v - vb), a1 = __shfl_sync(kFull, q1, v - vb);
+                for (int J0 = a0; J0 < a1; J0 += 32) {
+                    bool ok = false;
+                    if (J0 + lane < a1) {
+                        const float4 hj = bh[J0 + lane];
+                        ok = hj.w >= 0.f && boxes_close<true>(ci, hi, bc[J0 + lane], hj, box, inv_box, cut, cut2);
+                    }
+                    for (unsigned left = __ballot_sync(kFull, ok); left; left &= left - 1) {
+                        const int J = J0 + __ffs(left) - 1;
+                        const float4 cj = bc[J], hj = bh[J], xj = xs[J * 32 + lane];
+                        const float3 d = min_image(make_float3(cj.x - ci.x, cj.y - ci.y, cj.z - ci.z), box, inv_box);
+                        auto near = [&](float4 x, float sign, float4 h) {  // false for padding (NaN)
+                            const float gx = fmaxf(0.f, fabsf(d.x + sign * x.x) - h.x);
+                            const float gy = fmaxf(0.f, fabsf(d.y + sign * x.y) - h.y);
+                            const float gz = fmaxf(0.f, fabsf(d.z + sign * x.z) - h.z);
+                            return x.x == x.x && gx * gx + gy * gy + gz * gz < cut2;
+                        };
+                        const bool wide = hi.x + hj.x + cut >= 0.5f * box.x || hi.y + hj.y + cut >= 0.5f * box.y ||
+                                          hi.z + hj.z + cut >= 0.5f * box.z;
+                        if (!wide && !(__any_sync(kFull, near(xi, -1.f, hj)) && __any_sync(kFull, near(xj, 1.f, hi))))
+                            continue;
+                        if (lane == 0 && found < kMaxNeighbours) s_seg[warp][found] = J;
+                        ++found;
+                        upper += J >= I;
+                    }
+                }
+            }
         }
-        if (lane == 0) {
-            s_m = min(m, nb.cap);
-            nb.cnt[I] = min(m, nb.cap);
-            atomicMax(&nb.stats[0], s_col[columns] > kMaxCandidates ? kMaxNeighbours + 1 : m);
-            atomicAdd(&nb.stats[2], upper);
-            if (m > nb.cap || s_col[columns] > kMaxCandidates) atomicOr(nb.flags, ListFlags::kNeighbourOverflow);
+    }
+    if (lane == 0) {
+        s_cnt[warp] = found;
+        if (upper) atomicAdd(&nb.stats[2], upper);
+    }
+    __syncthreads();
+    int total = 0, before = 0;
+#pragma unroll
+    for (int w = 0; w < kBuildWarps; ++w) {
+        if (w < warp) before += s_cnt[w];
+        total += s_cnt[w];
+    }
+    for (int k = lane; k < min(found, kMaxNeighbours) && before + k < nb.cap; k += 32) sj[before + k] = s_seg[warp][k];
+    __syncthreads();
+    const int m = min(total, nb.cap);
+    if (tid < m) {  // by few warps: FP64 arithmetic
+        const int J = sj[tid];
+        const float4 ei = ext[I], ej = ext[J];
+        const float3 A = anchor_shift(ci, bc[J], bd);
+        const bool wrap = fabsf(A.x) + ei.x + ej.x + pad >= 0.5f * box.x || fabsf(A.y) + ei.y + ej.y + pad >= 0.5f * box.y ||
+                          fabsf(A.z) + ei.z + ej.z + pad >= 0.5f * box.z;
+        const float4 shift = make_float4(A.x, A.y, A.z, wrap ? 1.f : 0.f);
+        sA[tid] = shift;
+        nb.j[(size_t)I * nb.cap + tid] = J;
+        nb.shift[(size_t)I * nb.cap + tid] = shift;
+    }
+    for (int t = tid; t < 32 * m; t += kBuildThreads) px[t] = xs[sj[t >> 5] * 32 + (t & 31)];
+    if (tid == 0) {
+        nb.cnt[I] = min(total, nb.cap);
+        atomicMax(&nb.stats[0], total);
+        if (total > nb.cap) atomicOr(nb.flags, ListFlags::kNeighbourOverflow);
+    }
+    __syncthreads();
+    {
+        const float4 xi = xs[I * 32 + lane];
+        uint16_t* mask16 = reinterpret_cast<uint16_t*>(masks);
+        for (int it = warp; it < 2 * m; it += kBuildWarps) {
+            const int q = it >> 1;
+            const float4 A = sA[q];
+            const float4* p = px + 32 * q + 16 * (it & 1);
+            uint32_t hit = 0u;
+            if (A.w == 0.f) {
+#pragma unroll
+                for (int t = 0; t < 16; ++t)
+                    hit |= (norm2(anchored_sep(xi, p[t], make_float3(A.x, A.y, A.z))) < cut2 ? 1u : 0u) << t;
+            } else {
+                for (int t = 0; t < 16; ++t) {
+                    const float3 d = min_image(anchored_sep(xi, p[t], make_float3(A.x, A.y, A.z)), box, inv_box);
+                    hit |= (norm2(d) < cut2 ? 1u : 0u) << t;
+                }
+            }
+            if (sj[q] == I && (it & 1) == lane >> 4) hit &= ~(1u << (lane & 15));  // the bead itself
+            mask16[2 * (32 * q + lane) + (it & 1)] = (uint16_t)hit;
         }
     }
     __syncthreads();
-    const int m = s_m;
-    for (int t = tid; t < 32 * m; t += kBuildThreads) px[t] = xs[sj[t >> 5] * 32 + (t & 31)];
+    for (int e = e0 + warp; e < e1; e += kBuildWarps) {
+        const int ex = e == e0 + warp ? first : excluded_slot(e);
+        if (ex < 0) continue;
+        for (int q = 0; q < m; ++q)
+            if (sj[q] == ex >> 5) atomicAnd(&masks[32 * q + lane], ~(1u << (ex & 31)));
+    }
     __syncthreads();
     const int unit_cap = nb.list_groups * 4;
     for (int b = warp; b < 32; b += kBuildWarps) {
-        const int o = perm[I * 32 + b];
-        if (o < 0) {
+        if (perm[I * 32 + b] < 0) {
             if (lane == 0) nb.len[I * 32 + b] = 0;
             continue;
         }
-        const int e0 = ex_csr[o], e1 = ex_csr[o + 1];
-        auto excluded_slot = [&](int e) { return e < e1 && (ex_bits[e] & kTermLJR) ? slot[ex_j[e]] : -1; };
-        const int first = excluded_slot(e0 + lane);
-        const bool many = e1 - e0 > 32;
-        const float4 xi = xs[I * 32 + b];
+        uint16_t* const row = rows + warp * kListUnits * unit_cap;
+        const unsigned below = (1u << lane) - 1u;
         int cnt = 0;
-        for (int h = 0; h < m; h += 32) {
-            bool ok = false;
-            const int Jh = h + lane < m ? sj[h + lane] : -1;
-            if (Jh >= 0) {
-                const float4 A = sA[h + lane], hj = bh[Jh];
-                const float gx = fmaxf(0.f, fabsf(A.x - xi.x) - hj.x);
-                const float gy = fmaxf(0.f, fabsf(A.y - xi.y) - hj.y);
-                const float gz = fmaxf(0.f, fabsf(A.z - xi.z) - hj.z);
-                ok = A.w != 0.f || gx * gx + gy * gy + gz * gz < cut2;
-            }
-            // boxes that hold an excluded partner (every box when the row is long)
-            bool holds = many;
-            if (!many)
-                for (int e = 0; e < e1 - e0; ++e) {
-                    const int x = __shfl_sync(kFull, first, e);
-                    holds = holds || (x >= 0 && x >> 5 == Jh);
-                }
-            const unsigned hold_mask = __ballot_sync(kFull, holds);
-            for (unsigned left = __ballot_sync(kFull, ok); left; left &= left - 1) {
-                const int l = __ffs(left) - 1, q = h + l;
-                const float4 A = sA[q];
-                float3 d = anchored_sep(xi, px[32 * q + lane], make_float3(A.x, A.y, A.z));
-                if (A.w != 0.f) d = min_image(d, box, inv_box);
-                unsigned hits = __ballot_sync(kFull, norm2(d) < cut2);
-                const int J = sj[q];
-                if (J == I) hits &= ~(1u << b);
-                if (hold_mask >> l & 1u)
-                    for (int e = e0; e < e1; e += 32) {
-                        const int ex = e == e0 ? first : excluded_slot(e + lane);
-                        for (unsigned x = __ballot_sync(kFull, ex >= 0 && ex >> 5 == J); x; x &= x - 1)
-                            hits &= ~(1u << (__shfl_sync(kFull, ex, __ffs(x) - 1) & 31));
-                    }
-                if (hits >> lane & 1u) {
-                    const int k = cnt + __popc(hits & ((1u << lane) - 1u));
-                    if (k / kListUnits < unit_cap)
-                        nb.list[list_at(nb, I, k / kListUnits, kListUnits * b + k % kListUnits)] =
-                            (uint16_t)((32 * q + lane) << 3);
-                }
-                cnt += __popc(hits);
-            }
+#pragma unroll 4
+        for (int q = 0; q < m; ++q) {
+            const uint32_t word = masks[32 * q + b];
+            const int k = cnt + __popc(word & below);
+            if ((word >> lane & 1u) && k < kListUnits * unit_cap) row[k] = (uint16_t)((32 * q + lane) << 3);
+            cnt += __popc(word);
         }
+        __syncwarp();
+        uint16_t* const out = nb.list + list_at(nb, I, 0, kListUnits * b);
+        for (int k = lane; k < min(cnt, kListUnits * unit_cap); k += 32) {
+            const int p = k / kListUnits;  // list_at(nb, I, p, kListUnits * b + k % kListUnits)
+            out[((p >> 2) * kListThreads + k % kListUnits) * 4 + (p & 3)] = row[k];
+        }
+        __syncwarp();
         if (lane < kListUnits)  // fill up the unit's last group
             for (int k = unit_entries(cnt, lane); (k & 3) && k < unit_cap; ++k)
                 nb.list[list_at(nb, I, k, kListUnits * b + lane)] = (uint16_t)((32 * nb.cap) << 3);
@@ -2046,11 +2089,12 @@ NeighbourLists PlainContext::neighbour_lists() const {
     return nb;
 }
 
-// Shared memory of a pair-list block: staged positions and shifts, and for
-// the force kernel the Lennard-Jones parameters.
+// Shared memory of a pair-list block: staged positions and shifts, the Lennard-
+// Jones parameters for the force kernel, the hit masks for the build.
 size_t PlainContext::list_smem(bool same_sigma, bool build) const {
-    const size_t beads = 32 * (size_t)nbr_cap_ + 1;
-    return 16 * beads + 16 * ((size_t)nbr_cap_ + 1) + (build ? 0 : (same_sigma ? 8 : 16) * beads);
+    const size_t shifts = 16 * ((size_t)nbr_cap_ + 1), beads = 32 * (size_t)nbr_cap_ + 1;
+    if (build) return build_region(nbr_cap_, list_cap_ / 4) + shifts + 128 * (size_t)nbr_cap_;
+    return 16 * beads + shifts + (same_sigma ? 8 : 16) * beads;
 }
 
 void PlainContext::alloc_pair_lists() {
@@ -2064,7 +2108,9 @@ void PlainContext::alloc_pair_lists() {
     OCM_CK(cudaMemsetAsync(nbr_cnt_.p, 0, nc * sizeof(int32_t), stream_));
     OCM_CK(cudaMemsetAsync(list_len_.p, 0, nc * 32 * sizeof(int32_t), stream_));
     // the limit is the kernels', not this context's: always the largest
-    const int most = 32 * kMaxNeighbours + 1, bytes = 32 * most + 16 * (kMaxNeighbours + 1);
+    const int most = 32 * kMaxNeighbours + 1;
+    const int bytes = std::max(32 * most, build_region(kMaxNeighbours, 4 * kMaxNeighbours / 4) + 128 * kMaxNeighbours) +
+                      16 * (kMaxNeighbours + 1);
     const void* fns[] = {(const void*)k_forces_lists<true, false>,  (const void*)k_forces_lists<true, true>,
                          (const void*)k_forces_lists<false, false>, (const void*)k_forces_lists<false, true>,
                          (const void*)k_pair_lists};

@@ -170,6 +170,7 @@ class PlainContext {
     cudaStream_t stream_ = nullptr;
     std::map<int, cudaGraphExec_t> graphs_;
     bool positions_set_ = false;
+    bool dependent_launches_ = false;  // of the last force launch (plain_engine.cu)
     LangevinConsts lc_{};
     int cell_dims_[3] = {1, 1, 1};
     int num_sms_ = 1;

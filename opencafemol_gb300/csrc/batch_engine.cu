@@ -1406,6 +1406,50 @@ __global__ void k_batch_velocity_init(int n, long long off, const float* __restr
     vz[off + i] = s * g.z;
 }
 
+// State of one slot from and to a caller's arrays (load_state_device,
+// store_state_device).
+__global__ void k_load_state(int n, long long off, const double* __restrict__ x, const double* __restrict__ y,
+                             const double* __restrict__ z, const float* __restrict__ vx,
+                             const float* __restrict__ vy, const float* __restrict__ vz, double* bx, double* by,
+                             double* bz, float* bvx, float* bvy, float* bvz, BatchSys* rec,
+                             unsigned long long steps_done, unsigned long long steps_target) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        rec->steps_done = steps_done;
+        rec->steps_target = steps_target;
+        rec->status = 0;
+    }
+    if (i >= n) return;
+    bx[off + i] = x[i];
+    by[off + i] = y[i];
+    bz[off + i] = z[i];
+    bvx[off + i] = vx[i];
+    bvy[off + i] = vy[i];
+    bvz[off + i] = vz[i];
+}
+__global__ void k_store_state(int n, long long off, const BatchSys* __restrict__ rec, const double* __restrict__ bx,
+                              const double* __restrict__ by, const double* __restrict__ bz,
+                              const float* __restrict__ bvx, const float* __restrict__ bvy,
+                              const float* __restrict__ bvz, double* x, double* y, double* z, float* vx, float* vy,
+                              float* vz, float4* xq, float4* xlo, unsigned long long* step_base,
+                              unsigned long long steps) {
+    if (rec->status != 0) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *step_base += steps;
+    if (i >= n) return;
+    const double p[3] = {bx[off + i], by[off + i], bz[off + i]};
+    x[i] = p[0];
+    y[i] = p[1];
+    z[i] = p[2];
+    vx[i] = bvx[off + i];
+    vy[i] = bvy[off + i];
+    vz[i] = bvz[off + i];
+    const float h[3] = {__double2float_rn(p[0]), __double2float_rn(p[1]), __double2float_rn(p[2])};
+    xq[i] = make_float4(h[0], h[1], h[2], 0.f);
+    xlo[i] = make_float4(__double2float_rn(p[0] - (double)h[0]), __double2float_rn(p[1] - (double)h[1]),
+                         __double2float_rn(p[2] - (double)h[2]), 0.f);
+}
+
 // Persistent launch: as many CTAs as fit, each given an equal share of the
 // SM's shared memory (the state needs `smem`; the rest holds neighbour
 // lists).
@@ -2054,8 +2098,10 @@ void BatchEngine::launch(bool integrate, int k, const std::vector<int32_t>& orde
     if ((int64_t)smem > optin)
         throw Error(6, "[error] these systems need more shared memory than one SM offers; "
                        "create the batch with a smaller per-system bead limit");
-    OCM_CK(cudaMemcpyAsync(order_.p, order.data(), order.size() * sizeof(int32_t),
-                           cudaMemcpyHostToDevice, s));
+    if (order != order_up_) {  // a loop over the same systems keeps its claim order
+        OCM_CK(cudaMemcpyAsync(order_.p, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+        order_up_ = order;
+    }
     if (order_k)
         OCM_CK(cudaMemcpyAsync(order_k_.p, order_k->data(), order_k->size() * sizeof(int32_t),
                                cudaMemcpyHostToDevice, s));
@@ -2085,7 +2131,8 @@ void BatchEngine::run(int32_t k, bool sync) {
     OCM_CK(cudaSetDevice(device_));
     if (k <= 0) throw Error(1, "[error] steps per launch must be positive");
     // settle the previous launch first: list growth and systems that blew up
-    grow_lists();
+    // (a state loaded since then need not be waited for)
+    if (!settled_) grow_lists();
     std::vector<int32_t> order;
     for (int64_t s = 0; s < max_systems_; ++s)
         if (slots_[s].used && !slots_[s].failed && slots_[s].steps_done < slots_[s].steps_target)
@@ -2110,6 +2157,7 @@ void BatchEngine::run(int32_t k, bool sync) {
     OCM_CK(cudaMemcpy2DAsync(h_status_, sizeof(int), &sys_.p[0].status, sizeof(BatchSys),
                              sizeof(int), max_systems_, cudaMemcpyDeviceToHost, stream_));
     ran_ = true;
+    settled_ = false;
     for (size_t q = 0; q < order.size(); ++q) {
         Slot& S = slots_[order[q]];
         S.steps_done = std::min<uint64_t>(S.steps_target, S.steps_done + (uint64_t)ks[q]);
@@ -2147,46 +2195,31 @@ void BatchEngine::load_state_device(int64_t slot, const double* x, const double*
     OCM_CK(cudaSetDevice(device_));
     if (slot < 0 || slot >= max_systems_ || !slots_[slot].used) throw Error(1, "[error] invalid slot");
     if (steps_done > steps_target) throw Error(1, "[error] steps already done exceed the step target");
-    sync_steps();
+    grow_lists();  // settles the last launch
     Slot& S = slots_[slot];
     const int64_t n = S.n, o = S.bead_off;
-    cudaStream_t s = stream_;
-    OCM_CK(cudaMemcpyAsync(x_.p + o, x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(y_.p + o, y, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(z_.p + o, z, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vx_.p + o, vx, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vy_.p + o, vy, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vz_.p + o, vz, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    k_load_state<<<(int)((n + 127) / 128), 128, 0, stream_>>>((int)n, o, x, y, z, vx, vy, vz, x_.p, y_.p, z_.p, vx_.p,
+                                                              vy_.p, vz_.p, sys_.p + slot, steps_done, steps_target);
+    OCM_CK(cudaGetLastError());
     BatchSys& R = sys_host_[slot];
     R.steps_done = steps_done;
     R.steps_target = steps_target;
     R.status = 0;
-    BatchSys* dst = sys_.p + slot;
-    OCM_CK(cudaMemcpyAsync(&dst->steps_done, &R.steps_done, 2 * sizeof(unsigned long long),
-                           cudaMemcpyHostToDevice, s));
-    OCM_CK(cudaMemcpyAsync(&dst->status, &R.status, sizeof(int), cudaMemcpyHostToDevice, s));
-    OCM_CK(cudaStreamSynchronize(s));
     S.steps_done = steps_done;
     S.steps_target = steps_target;
     S.failed = false;
     h_status_[slot] = 0;
 }
 
-void BatchEngine::store_state_device(int64_t slot, double* x, double* y, double* z, float* vx, float* vy,
-                                     float* vz) {
+void BatchEngine::store_state_device(int64_t slot, double* x, double* y, double* z, float* vx, float* vy, float* vz,
+                                     float4* xq, float4* xlo, unsigned long long* step_base, uint64_t steps) {
     OCM_CK(cudaSetDevice(device_));
     if (slot < 0 || slot >= max_systems_ || !slots_[slot].used) throw Error(1, "[error] invalid slot");
-    sync_steps();
     const Slot& S = slots_[slot];
-    const int64_t n = S.n, o = S.bead_off;
-    cudaStream_t s = stream_;
-    OCM_CK(cudaMemcpyAsync(x, x_.p + o, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(y, y_.p + o, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(z, z_.p + o, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vx, vx_.p + o, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vy, vy_.p + o, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaMemcpyAsync(vz, vz_.p + o, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-    OCM_CK(cudaStreamSynchronize(s));
+    k_store_state<<<(int)((S.n + 127) / 128), 128, 0, stream_>>>((int)S.n, S.bead_off, sys_.p + slot, x_.p, y_.p, z_.p,
+                                                                 vx_.p, vy_.p, vz_.p, x, y, z, vx, vy, vz, xq, xlo,
+                                                                 step_base, steps);
+    OCM_CK(cudaGetLastError());
 }
 
 int32_t BatchEngine::slot_status(int64_t slot) {
@@ -2201,6 +2234,7 @@ int32_t BatchEngine::slot_status(int64_t slot) {
 void BatchEngine::grow_lists() {
     if (!ran_) return;
     sync_steps();
+    settled_ = true;
     for (int64_t s = 0; s < max_systems_; ++s) {
         if (!h_overflow_[s] || !slots_[s].used) continue;
         h_overflow_[s] = 0;

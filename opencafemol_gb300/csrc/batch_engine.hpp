@@ -81,10 +81,14 @@ class BatchEngine {
     // Device-to-device state exchange of one slot with buffers of the same
     // device (the plain context's one-system fast path): positions (FP64
     // SoA), velocities (FP32 SoA), the step counter and the step target.
-    // Both wait for the batch's stream; the copies are complete on return.
+    // One kernel each on the batch's stream, not waited for: the caller's
+    // arrays must be ready, and slot_status waits.  store writes nothing
+    // when the system blew up; it also refreshes the FP32 pair of every
+    // position and adds `steps` to the caller's step counter.
     void load_state_device(int64_t slot, const double* x, const double* y, const double* z, const float* vx,
                            const float* vy, const float* vz, uint64_t steps_done, uint64_t steps_target);
-    void store_state_device(int64_t slot, double* x, double* y, double* z, float* vx, float* vy, float* vz);
+    void store_state_device(int64_t slot, double* x, double* y, double* z, float* vx, float* vy, float* vz, float4* xq,
+                            float4* xlo, unsigned long long* step_base, uint64_t steps);
     void run(int32_t steps_per_launch, bool sync);
     void finished(int64_t* slots, int64_t cap, int64_t* n_out);
     void get_positions(int64_t slot, double* xyz);
@@ -144,6 +148,8 @@ class BatchEngine {
     cudaStream_t stream_ = nullptr, copy_stream_ = nullptr;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_copy_ = nullptr;
     bool ran_ = false;
+    bool settled_ = true;  // no launch since the last sync_steps
+    std::vector<int32_t> order_up_;  // the claim order that is on the device
     std::vector<Slot> slots_;
     RangeAllocator beads_, blob_, list_alloc_;
     DevBuf<double> x_, y_, z_;

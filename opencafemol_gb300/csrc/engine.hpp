@@ -241,6 +241,8 @@ class PlainContext {
     DevBuf<float> svx_, svy_, svz_;
     DevBuf<unsigned long long> sstep_;
     int32_t* h_flags_ = nullptr;  // pinned
+    double* h_energy_ = nullptr;  // pinned, kNumSlots
+    DevBuf<double> pack_;         // 3 * n, the interleaved host layout
 };
 
 // Many independent systems, each advanced inside one CTA's shared memory.

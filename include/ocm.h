@@ -301,8 +301,9 @@ int ocm_context_minimize_report(ocm_context* ctx, int32_t* reason, double* rms_f
 typedef struct ocm_context_stats {
     int64_t steps_done;
     int64_t list_builds;
-    int64_t tiles;            /* cluster-pair tiles in the current list */
-    int64_t masked_tiles;     /* tiles carrying exclusion masks */
+    int64_t tiles;            /* cluster-pair tiles in the current list (pairs of neighbour
+                               * clusters where per-bead lists take the tiles' place) */
+    int64_t masked_tiles;     /* tiles carrying exclusion masks (0 with per-bead lists) */
     int32_t rebuild_interval; /* steps between list builds */
     int32_t reordered;        /* 1 if beads are sorted into column clusters */
     double  skin;             /* nm */

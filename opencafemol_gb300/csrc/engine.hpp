@@ -145,6 +145,7 @@ class PlainContext {
     void alloc_pair_lists();
     void leave_pair_lists();
     void setup_charged_cells();
+    void layout_counters();
     void setup_columns(double width);
     BoxD box_d() const;
     float wrap_pad() const;
@@ -190,7 +191,7 @@ class PlainContext {
     // Per-bead pair lists of the Lennard-Jones terms instead of tiles
     bool pair_lists_ = false;
     int nbr_cap_ = 0, list_cap_ = 0;  // neighbour clusters per cluster, entries per unit
-    DevBuf<int32_t> nbr_cnt_, nbr_j_, list_len_, nbr_stats_;
+    DevBuf<int32_t> nbr_cnt_, nbr_j_, list_len_;
     DevBuf<float4> nbr_shift_, ljs_;
     DevBuf<uint16_t> list_;
 
@@ -216,14 +217,18 @@ class PlainContext {
     DevBuf<int32_t> mask_count_;
     // cluster order: columns in x-y, each sorted along z in thin slices
     double col_wmin_ = 1.0;
-    DevBuf<int32_t> cell_key_, cell_count_, cell_start_, cell_fill_, bucket_, col_start_;
+    DevBuf<int32_t> cell_key_, cell_start_, bucket_, col_start_;
+    // counters of a list build (layout_counters)
+    DevBuf<int32_t> zeroed_;
+    int32_t *cell_count_ = nullptr, *cell_fill_ = nullptr, *chg_count_ = nullptr, *chg_fill_ = nullptr,
+            *chg_stats_ = nullptr, *nbr_stats_ = nullptr;
     // exclusions
     DevBuf<int32_t> ex_start_, ex_j_;
     DevBuf<uint8_t> ex_bits_;
     // charged-pair list
-    DevBuf<int32_t> chg_idx_, chg_key_, chg_count_, chg_start_, chg_fill_;
+    DevBuf<int32_t> chg_idx_, chg_key_, chg_start_;
     DevBuf<float4> chg_sorted_;  // charged beads by cell: x, y, z, index bits
-    DevBuf<int32_t> chg_rows_, chg_len_, chg_stats_;  // rows, row lengths, {longest, entries}
+    DevBuf<int32_t> chg_rows_, chg_len_;  // rows, row lengths (chg_stats_: longest, entries)
     DevBuf<int32_t> ex_csr_;  // per-bead start of its exclusion row (n + 1)
     // bonded
     DevBuf<BondTerm> bonds_;

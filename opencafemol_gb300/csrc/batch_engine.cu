@@ -2234,7 +2234,6 @@ int32_t BatchEngine::slot_status(int64_t slot) {
 void BatchEngine::grow_lists() {
     if (!ran_) return;
     sync_steps();
-    settled_ = true;
     for (int64_t s = 0; s < max_systems_; ++s) {
         if (!h_overflow_[s] || !slots_[s].used) continue;
         h_overflow_[s] = 0;
@@ -2264,6 +2263,7 @@ void BatchEngine::grow_lists() {
                                cudaMemcpyHostToDevice, stream_));
         OCM_CK(cudaStreamSynchronize(stream_));
     }
+    settled_ = true;
 }
 
 void BatchEngine::finished(int64_t* out, int64_t cap, int64_t* n_out) {

@@ -94,6 +94,11 @@ constexpr int kClassGeneral = 2;
 constexpr int kBeadBytes[3] = {104, 112, 120};
 constexpr size_t kFixedBytes =
     (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kSplitMost + kSplitMost / 2 + 4 * kSortBuckets + 16;
+// Largest system of a quarter of a CTA, in launches of at least four systems
+// per CTA: a step of 60 beads makes about ten work items, so half a CTA's
+// eight warps wait for the second round of two of them.  1,400 peptides of
+// 30..80 beads: 2.04 -> 1.71 ms per 100 steps with the read-out.
+constexpr int kQuarterBeads = 96;
 // A force component beyond this (kJ/mol/nm) marks a blown-up system: far
 // above any physical coarse-grained force, and the bound of the plain
 // engine's fixed-point accumulators.
@@ -130,6 +135,7 @@ struct BatchArgs {
     uint32_t slots_enabled;
     size_t smem_bytes;           // dynamic shared memory of the launch
     int split_beads;             // a CTA splits into two groups at systems of at most this many beads (0: never)
+    int quarter_beads;           // and a group into two again at these (0: never)
     int split_bead_bytes;        // host side: shared-memory state bytes per bead (caps split_beads)
 };
 
@@ -1309,16 +1315,51 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     }
 }
 
+// A group of GT threads claims and advances systems with its own barrier,
+// shared memory and words, starting with order entry `first` (-1: with a
+// claim).  It returns -1 when no system is left, or the order entry of a
+// claimed system of at most smaller_beads beads (0: never), which it has not
+// run: the caller divides the group.
+template <int GT, int MODE, bool ENERGY, bool INTEGRATE>
+__device__ __forceinline__ int split_phase(const BatchArgs& a, int g, int gtid, int bar, unsigned char* gsmem,
+                                           size_t gbytes, int first, int smaller_beads, int& claim, int* move,
+                                           int& overflow, int& bad, double* energy, int& item) {
+    while (true) {
+        if (gtid == 0) {
+            claim = first >= 0 ? first : atomicAdd(a.head, 1);
+            move[0] = 0;
+            move[1] = 0;
+            overflow = 0;
+            bad = 0;
+        }
+        first = -1;
+        if (ENERGY && gtid < kNumSlots) energy[gtid] = 0.0;
+        bar_sync(bar, GT);
+        const int q = claim;
+        if (q >= a.n_order) return -1;
+        const int slot = a.order[q];
+        if (INTEGRATE && a.sys[slot].status != 0) {
+            bar_sync(bar, GT);
+            continue;
+        }
+        if (a.sys[slot].n <= smaller_beads) return q;
+        run_system<GT, MODE, ENERGY, INTEGRATE>(a, q, slot, gtid, bar, gsmem, gbytes, move, &overflow, &bad, energy,
+                                                &item);
+        bar_sync(bar, GT);
+    }
+}
+
 template <int THREADS, int MODE, bool ENERGY, bool INTEGRATE>
 __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    // per-group state (group 0 only until the split)
-    __shared__ int s_claim[2];
-    __shared__ int s_move[2][2];
-    __shared__ int s_overflow[2];
-    __shared__ int s_bad[2];
-    __shared__ double s_energy[2][kNumSlots];
-    __shared__ int s_item[2];
+    // per-group state: the whole CTA and the halves in 0 and 1 (the CTA's own
+    // until the split), the quarters in 2..5
+    __shared__ int s_claim[6];
+    __shared__ int s_move[6][2];
+    __shared__ int s_overflow[6];
+    __shared__ int s_bad[6];
+    __shared__ double s_energy[6][kNumSlots];
+    __shared__ int s_item[6];
     const int tid = threadIdx.x;
 
     // Whole-CTA phase: every claimed system runs on all THREADS threads
@@ -1358,40 +1399,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
 
     // Split phase, for the rest of the launch: two groups of THREADS / 2
     // threads, each with half of the shared memory and its own named barrier
-    // (1 + g), each claiming and advancing its own systems; no barrier spans
-    // both groups.  Group 0 starts with the system the CTA claimed (its words
-    // were reset at that claim).  A system's results do not depend on the
-    // threads that run it (the pair split depends on its bead count alone),
-    // so they do not depend on the split either.
-    constexpr int GT = THREADS / 2;
-    const int g = tid / GT, gtid = tid - g * GT;
-    const size_t half = (a.smem_bytes / 2) & ~(size_t)255;
-    unsigned char* gsmem = smem + (size_t)g * half;
-    bool first = g == 0;
-    while (true) {
-        if (!first) {
-            if (gtid == 0) {
-                s_claim[g] = atomicAdd(a.head, 1);
-                s_move[g][0] = 0;
-                s_move[g][1] = 0;
-                s_overflow[g] = 0;
-                s_bad[g] = 0;
-            }
-            if (ENERGY && gtid < kNumSlots) s_energy[g][gtid] = 0.0;
-            bar_sync(1 + g, GT);
-        }
-        const int q = first ? split_q : s_claim[g];
-        first = false;
-        if (q >= a.n_order) return;
-        const int slot = a.order[q];
-        if (INTEGRATE && a.sys[slot].status != 0) {
-            bar_sync(1 + g, GT);
-            continue;
-        }
-        run_system<GT, MODE, ENERGY, INTEGRATE>(a, q, slot, gtid, 1 + g, gsmem, half, s_move[g], &s_overflow[g],
-                                                &s_bad[g], s_energy[g], &s_item[g]);
-        bar_sync(1 + g, GT);
-    }
+    // (1 + half), each claiming and advancing its own systems; no barrier
+    // spans both groups.  Group 0 starts with the system the CTA claimed.  A
+    // system's results do not depend on the threads that run it (the pair
+    // split depends on its bead count alone), so they do not depend on the
+    // split either.
+    const int half = tid / (THREADS / 2);
+    const size_t half_bytes = (a.smem_bytes / 2) & ~(size_t)255;
+    const int next_q = split_phase<THREADS / 2, MODE, ENERGY, INTEGRATE>(
+        a, half, tid % (THREADS / 2), 1 + half, smem + (size_t)half * half_bytes, half_bytes, half == 0 ? split_q : -1,
+        a.quarter_beads, s_claim[half], s_move[half], s_overflow[half], s_bad[half], s_energy[half], s_item[half]);
+    if (next_q < 0) return;
+    // Quarters, for the smallest systems: each half leaves its phase by
+    // itself, with a claimed system that its first quarter starts with.
+    const int quarter = tid / (THREADS / 4), w = 2 + quarter;
+    const size_t quarter_bytes = (half_bytes / 2) & ~(size_t)255;
+    split_phase<THREADS / 4, MODE, ENERGY, INTEGRATE>(
+        a, quarter, tid % (THREADS / 4), 3 + quarter,
+        smem + (size_t)half * half_bytes + (size_t)(quarter & 1) * quarter_bytes, quarter_bytes,
+        (quarter & 1) == 0 ? next_q : -1, 0, s_claim[w], s_move[w], s_overflow[w], s_bad[w], s_energy[w], s_item[w]);
 }
 
 __global__ void k_batch_velocity_init(int n, long long off, const float* __restrict__ invm,
@@ -1503,6 +1529,13 @@ void launch_persistent(Fn fn, int threads, BatchArgs a, int max_grid, size_t sme
         a.split_beads = std::min(a.split_beads, fit);
     }
     const int grid = std::max(1, std::min(max_grid, num_sms * per_sm));
+    if (a.split_beads > 0 && a.n_order >= 4 * grid) {
+        // enough systems to divide a group once more, by the same rule
+        const size_t quarter = (((share / 2) & ~(size_t)255) / 2) & ~(size_t)255;
+        const int fit =
+            quarter > kFixedBytes ? (int)((quarter - kFixedBytes) / (size_t)a.split_bead_bytes) & ~31 : 0;
+        a.quarter_beads = std::min({kQuarterBeads, a.split_beads, fit});
+    }
     fn<<<grid, threads, share, s>>>(a);
     OCM_CK(cudaGetLastError());
 }

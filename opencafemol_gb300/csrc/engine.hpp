@@ -143,6 +143,7 @@ class PlainContext {
     size_t list_smem(bool same_sigma, bool build) const;
     int column_reach(float cut, int reach[2]) const;
     void alloc_pair_lists();
+    bool pair_list_terms() const;
     void leave_pair_lists();
     void setup_charged_cells();
     void layout_counters();

@@ -1826,23 +1826,12 @@ PlainContext::PlainContext(const SystemDesc& d, double temperature, double frict
             }
         }
     }
-    // Per-bead pair lists instead of tiles: both Lennard-Jones terms with
-    // arithmetic epsilons and the same excluded pairs, no interaction groups,
-    // the column layout, and Debye-Hueckel absent or on its charged rows.
-    {
-        const int tile_terms = cs.pc.terms & ~(charged_split_ ? kTermDH : 0);
-        bool same = true;
-        for (uint8_t b : cs.ex_bits) same = same && ((b & kTermLJR) != 0) == ((b & kTermLJA) != 0);
-        // (leave_pair_lists: a neighbourhood of more than kMaxNeighbours
-        // clusters or kMaxColumns columns does not fit a block)
-        pair_lists_ = reorder && tile_terms == (kTermLJR | kTermLJA) && same && !cs.pc.ljr_geometric &&
-                      !(cs.pc.uses_labels & (kTermLJR | kTermLJA));
-        if (pair_lists_) {
-            nbr_cap_ = 48;
-            list_cap_ = 24;
-            ljs_.alloc(np);
-            alloc_pair_lists();
-        }
+    pair_lists_ = pair_list_terms();
+    if (pair_lists_) {
+        nbr_cap_ = 48;
+        list_cap_ = 24;
+        ljs_.alloc(np);
+        alloc_pair_lists();
     }
     bonds_.upload(cs.bonds, s);
     angles_.upload(cs.angles, s);
@@ -2555,7 +2544,20 @@ void PlainContext::step(int64_t nsteps) {
     throw Error(4, "[error] step could not complete after repeated list rebuilds");
 }
 
-// Back to the tiles, for a system whose neighbourhoods do not fit a block.
+// Whether per-bead pair lists can take the tiles' place: both Lennard-Jones
+// terms with arithmetic epsilons and the same excluded pairs, no interaction
+// groups, the column layout, and Debye-Hueckel absent or on its charged rows
+// (which list options can take away: setup_charged_cells).
+bool PlainContext::pair_list_terms() const {
+    const int tile_terms = cs.pc.terms & ~(charged_split_ ? kTermDH : 0);
+    bool same = true;
+    for (uint8_t b : cs.ex_bits) same = same && ((b & kTermLJR) != 0) == ((b & kTermLJA) != 0);
+    return reorder && tile_terms == (kTermLJR | kTermLJA) && same && !cs.pc.ljr_geometric &&
+           !(cs.pc.uses_labels & (kTermLJR | kTermLJA));
+}
+
+// Back to the tiles, for a system whose neighbourhoods do not fit a block
+// (more than kMaxNeighbours clusters or kMaxColumns columns).
 void PlainContext::leave_pair_lists() {
     pair_lists_ = false;
     clear_graphs();
@@ -2566,6 +2568,8 @@ void PlainContext::set_list_options(int32_t interval, double sk) {
     if (interval > 0) rebuild_interval = interval;
     if (sk > 0) skin = sk;
     setup_charged_cells();  // cells must stay at least cutoff + skin wide
+    // the lists hold no Debye-Hueckel: without the charged rows the tiles do
+    pair_lists_ = list_.n > 0 && pair_list_terms();
     clear_graphs();
 }
 

@@ -722,6 +722,7 @@ constexpr int kMaxNeighbours = 128;  // so that an entry fits 16 bits
 constexpr int kMaxColumns = 512;     // columns a neighbourhood may span
 constexpr int kListUnits = 8;
 constexpr int kListThreads = 32 * kListUnits;
+constexpr int kMaxUnitEntries = 32 * kMaxNeighbours / kListUnits;  // every staged bead
 constexpr int kBuildThreads = 512;
 constexpr int kBuildWarps = kBuildThreads / 32;
 
@@ -2116,7 +2117,7 @@ void PlainContext::alloc_pair_lists() {
     OCM_CK(cudaMemsetAsync(list_len_.p, 0, nc * 32 * sizeof(int32_t), stream_));
     // the limit is the kernels', not this context's: always the largest
     const int most = 32 * kMaxNeighbours + 1;
-    const int bytes = std::max(32 * most, build_region(kMaxNeighbours, 4 * kMaxNeighbours / 4) + 128 * kMaxNeighbours) +
+    const int bytes = std::max(32 * most, build_region(kMaxNeighbours, kMaxUnitEntries / 4) + 128 * kMaxNeighbours) +
                       16 * (kMaxNeighbours + 1);
     const void* fns[] = {(const void*)k_forces_lists<true, false>,  (const void*)k_forces_lists<true, true>,
                          (const void*)k_forces_lists<false, false>, (const void*)k_forces_lists<false, true>,
@@ -2266,8 +2267,9 @@ void PlainContext::ensure_capacity() {
             }
             // a few neighbours and 20% of list entries to spare
             const int want_n = std::min(kMaxNeighbours, (nbr[0] + 3) / 4 * 4 + 4);
-            const int want_l = (nbr[1] * 3 / 2 + 4 + 3) / 4 * 4;
-            if (nbr[0] > nbr_cap_ || (nbr[0] + 2 > nbr_cap_ && nbr_cap_ < want_n) || nbr[1] * 6 / 5 + 2 > list_cap_) {
+            const int want_l = std::min(kMaxUnitEntries, (nbr[1] * 3 / 2 + 4 + 3) / 4 * 4);
+            if (nbr[0] > nbr_cap_ || (nbr[0] + 2 > nbr_cap_ && nbr_cap_ < want_n) ||
+                (nbr[1] * 6 / 5 + 2 > list_cap_ && list_cap_ < want_l)) {
                 nbr_cap_ = std::max(nbr_cap_, want_n);
                 list_cap_ = std::max(list_cap_, want_l);
                 alloc_pair_lists();
@@ -2528,7 +2530,7 @@ void PlainContext::step(int64_t nsteps) {
                 leave_pair_lists();
             } else {
                 if (flags & ListFlags::kNeighbourOverflow) nbr_cap_ = std::min(kMaxNeighbours, nbr_cap_ + 8);
-                else list_cap_ += 4 + list_cap_ / 16 * 4;
+                else list_cap_ = std::min(kMaxUnitEntries, list_cap_ + 4 + list_cap_ / 16 * 4);
                 alloc_pair_lists();
             }
         }

@@ -66,3 +66,31 @@ def test_repeated_runs_are_bit_identical(gpu):
         ctx.step(120)
         out.append((ctx.getPositions(), ctx.getVelocities()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+def test_globule_with_nearly_every_bead_in_range(gpu):
+    """3,007 beads in a ball of 4.2 nm under a 4 nm cutoff: about 375 entries
+    per unit, so the head-room reaches the most that a unit can hold (every
+    staged bead, 512), and that is where it stops."""
+    from opencafemol_gb300 import synth
+    from oracle import oracle
+    spec = synth.hps_slab(31, 97, (20.0, 20.0, 20.0), slab_width=18.0, seed=9, hps_cutoff=4.0)
+    spec.dh = None
+    side = 0.47 * np.arange(-10, 11)
+    grid = np.array([(x, y, z) for a, z in enumerate(side) for b, y in enumerate(side[:: 1 - 2 * (a % 2)])
+                     for x in side[:: 1 - 2 * (b % 2)]])  # neighbours in the chain are neighbours in space
+    r = np.linalg.norm(grid, axis=1)
+    ball = grid[np.sort(np.argsort(r, kind="stable")[: spec.n])]
+    spec.pos = (10.0 + ball + np.random.default_rng(4).normal(scale=0.01, size=ball.shape)).astype(np.float32).astype(np.float64)
+    spec.bond_v0 = np.linalg.norm(np.diff(spec.pos, axis=0), axis=1)[spec.bonds[:, 0]]
+    assert (np.linalg.norm(spec.pos - 10.0, axis=1) < 4.25).mean() > 0.95  # partners of the middle bead
+    system = synth.build_system(spec)
+    ctx = gpu.Context(system, gpu.LangevinIntegrator(spec.temperature, 5.0, 0.001, 7))
+    ctx.setPositions(spec.pos)
+    f, _ = ctx.getState(energy=False)
+    f_ref, _ = oracle.evaluate(spec)
+    assert rel_force_err(f, f_ref) <= FORCE_TOL
+    st = ctx.stats()
+    assert st["masked_tiles"] == 0 and st["tiles"] > 0  # the lists, not the tiles
+    ctx.step(20)
+    assert np.all(np.isfinite(ctx.getPositions()))

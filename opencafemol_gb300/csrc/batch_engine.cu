@@ -1798,39 +1798,6 @@ void check_batchable(const CompiledSystem& c, int nmax) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-int64_t RangeAllocator::alloc(int64_t size, int64_t align) {
-    if (size <= 0) size = 1;
-    for (auto it = free_.begin(); it != free_.end(); ++it) {
-        const int64_t off = it->first, sz = it->second;
-        const int64_t a = align_up(off, align);
-        if (a + size <= off + sz) {
-            free_.erase(it);
-            if (a > off) free_[off] = a - off;
-            if (a + size < off + sz) free_[a + size] = off + sz - (a + size);
-            return a;
-        }
-    }
-    return -1;
-}
-
-void RangeAllocator::release(int64_t off, int64_t size) {
-    if (size <= 0) size = 1;
-    auto it = free_.emplace(off, size).first;
-    auto next = std::next(it);
-    if (next != free_.end() && it->first + it->second == next->first) {
-        it->second += next->second;
-        free_.erase(next);
-    }
-    if (it != free_.begin()) {
-        auto prev = std::prev(it);
-        if (prev->first + prev->second == it->first) {
-            prev->second += it->second;
-            free_.erase(it);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 BatchEngine::BatchEngine(int device, int64_t max_systems, int64_t max_beads, int32_t nmax)
     : device_(device), max_systems_(max_systems), max_beads_(max_beads) {
     int count = 0;
@@ -2269,20 +2236,15 @@ void BatchEngine::grow_lists() {
     sync_steps();
     for (int64_t s = 0; s < max_systems_; ++s) {
         if (!h_overflow_[s] || !slots_[s].used) continue;
-        h_overflow_[s] = 0;
+        h_overflow_[s] = 0;  // also when the growth below fails: the run after the error goes on with the scan
         Slot& S = slots_[s];
         BatchSys R = sys_host_[s];
         auto grown = [](int cap, int limit) { return std::min((int)align_up(cap * 3 / 2 + 8, 4), limit); };
         R.maxn = grown(R.maxn, unit_capacity_limit(R.n, pair_split(R.n, split_units(R.cls))));
         if (R.nq) R.maxq = grown(R.maxq, unit_capacity_limit(R.nq, pair_split(R.nq, charged_units(R.cls))));
         const int64_t size = list_entries(R);
-        list_alloc_.release(S.list_off, S.list_size);
-        const int64_t off = list_alloc_.alloc(size, 64);
-        if (off < 0) {
-            const int64_t back = list_alloc_.alloc(S.list_size, 64);
-            (void)back;
-            throw Error(3, "[error] batch neighbour-list memory exhausted while growing a list");
-        }
+        const int64_t off = list_alloc_.regrow(S.list_off, S.list_size, size, 64);
+        if (off < 0) throw Error(3, "[error] batch neighbour-list memory exhausted while growing a list");
         S.list_off = off;
         S.list_size = size;
         R.list_off = off;

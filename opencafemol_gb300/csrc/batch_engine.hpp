@@ -8,11 +8,11 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <map>
 #include <vector>
 
 #include "engine.hpp"
 #include "host_system.hpp"
+#include "range_allocator.hpp"
 
 namespace ocm {
 
@@ -49,23 +49,6 @@ struct BatchSys {
     PairConsts pc;
     LangevinConsts lc;
     unsigned long long steps_done, steps_target;
-};
-
-// First-fit range allocator (units are arbitrary).
-class RangeAllocator {
-  public:
-    explicit RangeAllocator(int64_t cap = 0) { reset(cap); }
-    void reset(int64_t cap) {
-        cap_ = cap;
-        free_.clear();
-        if (cap > 0) free_[0] = cap;
-    }
-    int64_t alloc(int64_t size, int64_t align = 1);  // -1 when full
-    void release(int64_t off, int64_t size);
-    int64_t capacity() const { return cap_; }
-  private:
-    int64_t cap_ = 0;
-    std::map<int64_t, int64_t> free_;  // offset -> size
 };
 
 class BatchEngine {

@@ -91,7 +91,7 @@ constexpr int kClassGeneral = 2;
 // and the part that does not grow with the bead count (the dummy bead, the
 // cluster boxes and carries, the unit counts of small systems, the sort
 // buckets, alignment).
-constexpr int kBeadBytes[3] = {104, 112, 120};
+constexpr int kBeadBytes[3] = {104, 112, 108};  // by class
 constexpr size_t kFixedBytes =
     (size_t)(32 + 36) * kMaxClusters + 16 + 2 * kSplitMost + kSplitMost / 2 + 4 * kSortBuckets + 16;
 // Largest system of a quarter of a CTA, in launches of at least four systems
@@ -738,8 +738,11 @@ __device__ __forceinline__ void dh_pair(float4 xi, float4 xj, float qk, float qj
     if (ENERGY && in) ea.e[kSlotDH] += 0.5 * (double)(qq * (ex * rinv - pc.dh_corr));
 }
 
+// .w of a position is the bead's excluded-volume radius, p its charge,
+// repulsive epsilon and sigma and attractive epsilon, sg its attractive
+// sigma.
 template <bool ENERGY>
-__device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 p0i, float4 p0j, float4 p1i, float4 p1j,
+__device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 pi, float4 pj, float sgi, float sgj,
                                              uint32_t bits, const PairConsts& pc, float3& fa, EnergyAcc& ea) {
     const float3 nobox = make_float3(0.f, 0.f, 0.f);
     const float3 d = separation<false>(xi, xj, nobox, nobox);
@@ -747,7 +750,9 @@ __device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 p0i, f
     const bool in = r2 < pc.list_rc2;
     PairEnergy e;
     e.zero();
-    float sc = pair_scalar<15, ENERGY>(in ? r2 : pc.list_rc2, p0i, p0j, p1i, p1j, bits, pc, e);
+    float sc = pair_scalar<15, ENERGY>(in ? r2 : pc.list_rc2, make_float4(xi.w, pi.x, pi.y, pi.z),
+                                       make_float4(xj.w, pj.x, pj.y, pj.z), make_float4(pi.w, sgi, 0.f, 0.f),
+                                       make_float4(pj.w, sgj, 0.f, 0.f), bits, pc, e);
     sc = in ? sc : 0.f;
     sub_force(fa, sc, d);
     if (ENERGY && in) {
@@ -761,10 +766,11 @@ __device__ __forceinline__ void general_pair(float4 xi, float4 xj, float4 p0i, f
 
 // Per-bead parameters of the pair terms as staged in shared memory.
 struct PairParams {
-    const float4 *p0, *p1;  // General
-    const uint32_t* lab;    // General
-    const float2* le;       // Hps
-    const float* q;         // Go and Hps: charges
+    const float4* p;      // General (general_pair)
+    const float* sg;      // General
+    const uint32_t* lab;  // General
+    const float2* le;     // Hps
+    const float* q;       // Go and Hps: charges
 };
 
 // Main force on bead i from the cnt entries of column col, four entries at a
@@ -798,19 +804,21 @@ __device__ __forceinline__ float3 main_list(int i, int col, int cnt, const UnitL
             for (int u = 0; u < 4; ++u) hps_pair<ENERGY>(xi, xj[u], lei, lej[u], pc, f, ea);
         });
     } else {
-        const float4 p0i = P.p0[i], p1i = P.p1[i];
+        const float4 pi = P.p[i];
+        const float sgi = P.sg[i];
         list_walk(L, col, cnt, [&](uint2 e) {
-            float4 xj[4], p0j[4], p1j[4];
+            float4 xj[4], pj[4];
+            float sgj[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int j = (int)(entry_of(e, u) & 2047u);
                 xj[u] = sx[j];
-                p0j[u] = P.p0[j];
-                p1j[u] = P.p1[j];
+                pj[u] = P.p[j];
+                sgj[u] = P.sg[j];
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                general_pair<ENERGY>(xi, xj[u], p0i, p0j[u], p1i, p1j[u], (entry_of(e, u) >> 11) | excl_all, pc, f, ea);
+                general_pair<ENERGY>(xi, xj[u], pi, pj[u], sgi, sgj[u], (entry_of(e, u) >> 11) | excl_all, pc, f, ea);
         });
     }
     return f;
@@ -861,7 +869,7 @@ __device__ __forceinline__ float3 main_scan(int i, int j0, int j1, const float4*
             if (CLS == kClassGeneral) {
                 bits |= label_bits<true>(P.lab[i], P.lab[j], pc);
                 if ((bits & present) == present) continue;
-                general_pair<ENERGY>(xi, sx[j], P.p0[i], P.p0[j], P.p1[i], P.p1[j], bits | excl_all, pc, f, ea);
+                general_pair<ENERGY>(xi, sx[j], P.p[i], P.p[j], P.sg[i], P.sg[j], bits | excl_all, pc, f, ea);
             } else {
                 if (bits & drop) continue;
                 if (CLS == kClassGo) exv_pair<ENERGY>(xi, sx[j], pc, f, ea);
@@ -940,7 +948,8 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     float* sv = reinterpret_cast<float*>(carve(12 * (size_t)ns));
     float* sim = reinterpret_cast<float*>(carve(4 * (size_t)ns));
     float* sref = reinterpret_cast<float*>(carve(12 * (size_t)ns));
-    float4 *sp0 = nullptr, *sp1 = nullptr;
+    float4* sp = nullptr;
+    float* ssg = nullptr;
     uint32_t* slab = nullptr;
     float *fq = nullptr, *sq = nullptr;
     float2* sle = nullptr;
@@ -949,8 +958,8 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
         sq = reinterpret_cast<float*>(carve(4 * (size_t)ns));
         if (MODE != kClassGo && cls == kClassHps) sle = reinterpret_cast<float2*>(carve(8 * (size_t)ns));
     } else {
-        sp0 = reinterpret_cast<float4*>(carve(16 * (size_t)ns));
-        sp1 = reinterpret_cast<float4*>(carve(16 * (size_t)ns));
+        sp = reinterpret_cast<float4*>(carve(16 * (size_t)ns));
+        ssg = reinterpret_cast<float*>(carve(4 * (size_t)ns));
         slab = reinterpret_cast<uint32_t*>(carve(4 * (size_t)ns));
     }
     float4* bc = reinterpret_cast<float4*>(carve(16 * (size_t)nt));
@@ -1035,15 +1044,17 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
             if (MODE != kClassGo && cls == kClassHps)
                 sle[b] = make_float2(excl_all & kTermLJR ? 0.f : 0.5f * p0.z, excl_all & kTermLJA ? 0.f : 0.5f * gp1[b].x);
             if (!plain_cls) {
-                sp0[b] = p0;
-                sp1[b] = gp1[b];
+                const float4 p1 = gp1[b];
+                sp[b] = make_float4(p0.y, p0.z, p0.w, p1.x);
+                ssg[b] = p1.y;
                 slab[b] = glab[b];
             }
         } else {
             sx[b] = make_float4(nan, nan, nan, 0.f);
             sim[b] = 0.f;
             if (!plain_cls) {
-                sp0[b] = sp1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                sp[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                ssg[b] = 0.f;
                 slab[b] = 0xffffffffu;
             }
         }
@@ -1077,7 +1088,7 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     const float half_skin2 = 0.25f * R.skin * R.skin;
     bool use_scan = false;
     bool need_build = pairs_on;
-    const PairParams pp{sp0, sp1, slab, sle, sq};
+    const PairParams pp{sp, ssg, slab, sle, sq};
     int builds = 0;
     int st_done = 0;
     EnergyAcc ea;
@@ -1812,7 +1823,7 @@ BatchEngine::BatchEngine(int device, int64_t max_systems, int64_t max_beads, int
     OCM_CK(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device));
     int optin = 0;
     OCM_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    if ((int64_t)smem_bytes(nmax_, kClassGo) > optin)
+    if ((int64_t)smem_bytes(nmax_, kBeadBytes[kClassGo]) > optin)
         throw Error(6, "[error] per-system bead limit does not fit in shared memory");
     OCM_CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     OCM_CK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
@@ -1865,8 +1876,8 @@ BatchEngine::~BatchEngine() {
     if (copy_stream_) cudaStreamDestroy(copy_stream_);
 }
 
-// Shared memory of the per-system state of a class.
-size_t BatchEngine::smem_bytes(int nmax, int cls) const { return (size_t)nmax * kBeadBytes[cls] + kFixedBytes; }
+// Shared memory of the per-system state.
+size_t BatchEngine::smem_bytes(int nmax, int bead_bytes) const { return (size_t)nmax * bead_bytes + kFixedBytes; }
 
 int64_t BatchEngine::footprint(const SystemDesc& d) {
     CompiledSystem c = compile_system(d);
@@ -2085,13 +2096,14 @@ int64_t BatchEngine::admit(const SystemDesc& d, const double* pos, const double*
 
 void BatchEngine::launch(bool integrate, int k, const std::vector<int32_t>& order, cudaStream_t s,
                          const std::vector<int32_t>* order_k, uint32_t slots_enabled) {
-    int cls = kClassGo;
+    int cls = kClassGo, bead_bytes = 0;
     size_t bonded_max = 0;
     for (int32_t q : order) {
         cls = std::max(cls, slots_[q].cls);
+        bead_bytes = std::max(bead_bytes, kBeadBytes[slots_[q].cls]);
         bonded_max = std::max(bonded_max, (size_t)sys_host_[q].bonded_bytes);
     }
-    const size_t smem = smem_bytes(nmax_, cls);
+    const size_t smem = smem_bytes(nmax_, bead_bytes);
     const size_t want = list_smem_kib_ >= 0 ? smem + bonded_max + (size_t)list_smem_kib_ * 1024 : 0;
     int optin = 0;
     OCM_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
@@ -2123,7 +2135,7 @@ void BatchEngine::launch(bool integrate, int k, const std::vector<int32_t>& orde
     a.bead_order = bead_order_.p;
     a.slots_enabled = slots_enabled;
     a.split_beads = integrate ? split_beads_ : 0;
-    a.split_bead_bytes = kBeadBytes[cls];
+    a.split_bead_bytes = bead_bytes;
     launch_batch(cls, threads_, a, (int)order.size(), smem, s, integrate, num_sms_, want);
 }
 

@@ -120,7 +120,7 @@ class BatchEngine {
     // the kernel's per-step time grows with n, with a floor set by the
     // per-step barriers of small systems.
     static double step_cost(int64_t n) { return (double)std::max<int64_t>(n, 150); }
-    size_t smem_bytes(int nmax, int cls) const;
+    size_t smem_bytes(int nmax, int bead_bytes) const;
 
     int device_;
     int64_t max_systems_, max_beads_;

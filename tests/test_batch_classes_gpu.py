@@ -105,3 +105,18 @@ def test_overflow_scan_is_bit_identical(gpu, kind, n):
         b.run(30)
         out.append((b.positions(slot), b.velocities(slot)))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("kind", ["hps", "general"])
+def test_bead_limit_of_a_batch(gpu, kind):
+    """A batch for up to 1,888 beads per system takes a system of any class,
+    the largest included."""
+    from opencafemol_gb300 import synth
+    b = gpu.Batch(max_systems=2, max_total_beads=4096, max_beads_per_system=1888)
+    for n in (60, 1888):
+        spec = _chain(kind, n, 90 + n)
+        system = synth.build_system(spec)
+        slot = b.admit(system, spec.pos, seed=1, n_steps=5)
+        _check_state(b, slot, system, spec)
+    b.run(5)
+    assert all(b.status(s) == 0 and b.steps_done(s) == 5 for s in range(2))

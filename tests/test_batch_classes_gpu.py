@@ -120,3 +120,43 @@ def test_bead_limit_of_a_batch(gpu, kind):
         _check_state(b, slot, system, spec)
     b.run(5)
     assert all(b.status(s) == 0 and b.steps_done(s) == 5 for s in range(2))
+
+
+@pytest.mark.parametrize("terms", ["all", "wca_exv", "uniform_dh", "lja"])
+@pytest.mark.parametrize("n", [7, 65, 256, 600])
+def test_general_terms(gpu, terms, n):
+    """The General class with every pair term at once and with subsets (each
+    term is a block of its own in the inner loop): forces, energies and the
+    groups one at a time; the scan gives the list's bits."""
+    from opencafemol_gb300 import synth
+    spec = _chain("go", n, 700 + n)
+    rng = np.random.default_rng(n)
+    side = np.zeros(n, np.int8)
+    side[: max(1, n // 2)] |= 1
+    side[n // 3:] |= 2
+    if terms in ("all", "lja"):
+        sig = rng.uniform(0.35, 0.45, n)
+        spec.lja = synth.PairTerm(ratio=2.0 / np.sort(sig)[-2:].mean(), p0=rng.uniform(0.0, 0.8, n), p1=sig, ign_bond=2)
+    if terms == "all":
+        spec.ljr = synth.PairTerm(ratio=4.0, p0=np.full(n, 0.8), p1=rng.uniform(0.35, 0.45, n), ign_bond=1)
+    elif terms == "lja":
+        spec.exv = spec.dh = None
+    elif terms == "wca_exv":
+        spec.dh = None
+        spec.ljr = synth.PairTerm(ratio=0.0, p0=rng.uniform(0.3, 1.5, n), p1=rng.uniform(0.35, 0.55, n), kind="wca",
+                                  ign_bond=1)
+    else:
+        spec.exv = None
+        spec.lja = synth.PairTerm(ratio=3.0, p0=np.full(n, 0.6), p1=np.full(n, 0.4), kind="uniform", side=side, ign_bond=1)
+    system = synth.build_system(spec)
+    b = gpu.Batch(max_systems=2, max_total_beads=2048, max_beads_per_system=1024)
+    slot = b.admit(system, spec.pos, seed=1, n_steps=1)
+    _check_state(b, slot, system, spec)
+    f, _ = b.state(slot)
+    parts = sum(b.state(slot, groups=1 << g)[0] for g in range(len(system.group_names())))
+    assert np.allclose(parts, f, rtol=0, atol=1e-5 * max(1.0, np.abs(f).max()))
+    straight = np.zeros((n, 3))
+    straight[:, 0] = 0.38 * np.arange(n)  # too short lists for the coil: the scan
+    other = b.admit(system, straight, seed=1, n_steps=1)
+    b.set_positions_many([other], spec.pos)
+    assert np.array_equal(b.state(other)[0], f)

@@ -683,10 +683,13 @@ __device__ __forceinline__ void exv_pair(float4 xi, float4 xj, const PairConsts&
 // Both Lennard-Jones terms; .w of a position is half the bead's sigma, le
 // half its repulsive and attractive epsilon.  Inside the core (r <= 2^(1/6)
 // sigma) the repulsive term acts and the attractive one is flat, outside the
-// attractive one alone, so one power form serves both.
+// attractive one alone, so one power form serves both.  Evaluations of some
+// groups alone (ENERGY) may switch the terms off: zero epsilons do that for
+// the attraction, but in the core 0 times an overflowed power would be NaN,
+// hence rep_on for the repulsion.
 template <bool ENERGY>
-__device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float2 lej, const PairConsts& pc, float3& f,
-                                         EnergyAcc& ea) {
+__device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float2 lej, bool rep_on, const PairConsts& pc,
+                                         float3& f, EnergyAcc& ea) {
     const float3 d = make_float3(__fsub_rn(xj.x, xi.x), __fsub_rn(xj.y, xi.y), __fsub_rn(xj.z, xi.z));
     const float r2 = norm2(d);
     const bool in = r2 < pc.lja_rc2;
@@ -701,6 +704,7 @@ __device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float
     const float er = __fadd_rn(lei.x, lej.x), el = __fadd_rn(lei.y, lej.y);
     const float t = __fmul_rn(__fmul_rn(24.f, ri), __fmaf_rn(2.f, s12, -s6));
     float s = __fmul_rn(core ? er : el, t);
+    if (ENERGY && core && !rep_on) s = 0.f;
     const float r = __fmul_rn(r2, rinv);
     float sw = 1.f;
     if (r > pc.lja_rs) {
@@ -717,7 +721,7 @@ __device__ __forceinline__ void hps_pair(float4 xi, float4 xj, float2 lei, float
     sub_force(f, in ? s : 0.f, d);
     if (ENERGY && in) {
         const float e4 = 4.f * (s12 - s6);
-        if (core) ea.e[kSlotLJR] += 0.5 * (double)(er * (e4 + 1.f));
+        if (core && rep_on) ea.e[kSlotLJR] += 0.5 * (double)(er * (e4 + 1.f));
         ea.e[kSlotLJA] += 0.5 * (double)((core ? -el : el * e4) * sw);
     }
 }
@@ -851,6 +855,7 @@ struct PairParams {
     const float* sg;      // General
     const uint32_t* lab;  // General
     const float2* le;     // Hps
+    bool rep_on;          // Hps: the repulsive term is evaluated
     const float* q;       // Go and Hps: charges
 };
 
@@ -882,7 +887,7 @@ __device__ __forceinline__ float3 main_list(int i, int col, int cnt, const UnitL
                 lej[u] = P.le[entry_of(e, u) >> 4];
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) hps_pair<ENERGY>(xi, xj[u], lei, lej[u], pc, f, ea);
+            for (int u = 0; u < 4; ++u) hps_pair<ENERGY>(xi, xj[u], lei, lej[u], P.rep_on, pc, f, ea);
         });
     } else {
         const float4 pi = P.p[i];
@@ -957,7 +962,7 @@ __device__ __forceinline__ float3 main_scan(int i, int j0, int j1, const float4*
             } else {
                 if (bits & drop) continue;
                 if (CLS == kClassGo) exv_pair<ENERGY>(xi, sx[j], pc, f, ea);
-                else hps_pair<ENERGY>(xi, sx[j], P.le[i], P.le[j], pc, f, ea);
+                else hps_pair<ENERGY>(xi, sx[j], P.le[i], P.le[j], P.rep_on, pc, f, ea);
             }
         }
     }
@@ -1172,7 +1177,7 @@ __device__ __forceinline__ void run_system(const BatchArgs& a, int q, int slot, 
     const float half_skin2 = 0.25f * R.skin * R.skin;
     bool use_scan = false;
     bool need_build = pairs_on;
-    const PairParams pp{sp, ssg, slab, sle, sq};
+    const PairParams pp{sp, ssg, slab, sle, !(excl_all & kTermLJR), sq};
     int builds = 0;
     int st_done = 0;
     EnergyAcc ea;

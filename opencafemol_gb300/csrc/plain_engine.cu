@@ -1283,10 +1283,13 @@ __global__ void __launch_bounds__(kForceThreads) k_forces(ForceArgs a) {
 // Inside its core (r <= 2^(1/6) sigma) a term's repulsive part acts and its
 // attractive part is flat; outside it the attractive part acts alone.  With
 // one sigma for both terms (SAME) one power form serves both, with the bits
-// of the general form.  Every operation is rounded by itself.
+// of the general form.  Every operation is rounded by itself.  rep_on: the
+// repulsive term is evaluated; only the ENERGY form looks at it, which serves
+// the evaluations of some groups alone (a zero epsilon times an overflowed
+// power in the core would be NaN).
 template <bool SAME, bool ENERGY>
-__device__ __forceinline__ void lj_pair(float3 d, float hi, float hj, float4 lei, float4 lej, const PairConsts& pc,
-                                        float3& f, float& er_sum, float& ea_sum) {
+__device__ __forceinline__ void lj_pair(float3 d, float hi, float hj, float4 lei, float4 lej, bool rep_on,
+                                        const PairConsts& pc, float3& f, float& er_sum, float& ea_sum) {
     const float r2 = norm2(d);
     const bool in_r = r2 < pc.ljr_rc2, in_a = SAME ? in_r : r2 < pc.lja_rc2;
     const float rinv = rsqrtf(r2);
@@ -1311,7 +1314,7 @@ __device__ __forceinline__ void lj_pair(float3 d, float hi, float hj, float4 lei
     } else {
         ta = powers(__fadd_rn(lei.z, lej.z), a6, a12, acore);
     }
-    float rep = core ? __fmul_rn(er, t) : 0.f;
+    float rep = core && (!ENERGY || rep_on) ? __fmul_rn(er, t) : 0.f;
     float att = acore ? 0.f : __fmul_rn(el, ta);
     const float r = __fmul_rn(r2, rinv);
     float sw = 1.f;
@@ -1332,7 +1335,7 @@ __device__ __forceinline__ void lj_pair(float3 d, float hi, float hj, float4 lei
     f.y = __fmaf_rn(-s, d.y, f.y);
     f.z = __fmaf_rn(-s, d.z, f.z);
     if (ENERGY) {
-        if (in_r && core) er_sum += er * (4.f * (s12 - s6) + 1.f);
+        if (in_r && core && rep_on) er_sum += er * (4.f * (s12 - s6) + 1.f);
         if (in_a) ea_sum += (acore ? -el : el * (4.f * (a12 - a6))) * sw;
     }
 }
@@ -1408,7 +1411,7 @@ __global__ void __launch_bounds__(kListThreads, 4) k_forces_lists(ForceArgs a) {
         for (int u = 0; u < 4; ++u) {
             float3 d = anchored_sep(xi, xj[u], make_float3(A[u].x, A[u].y, A[u].z));
             if (wrap && A[u].w != 0.f) d = min_image(d, a.box, a.inv_box);
-            lj_pair<SAME, ENERGY>(d, pi.x, xj[u].w, lei, lej[u], a.pc, f, er4, ea4);
+            lj_pair<SAME, ENERGY>(d, pi.x, xj[u].w, lei, lej[u], !(a.excl_all & kTermLJR), a.pc, f, er4, ea4);
         }
         if (ENERGY) {
             er += (double)er4;
@@ -2195,8 +2198,9 @@ void PlainContext::launch_forces(cudaStream_t s, bool energy, uint32_t slots_ena
     if (pair_lists_) {
         const bool same = cs.lj_same_sigma && cs.pc.ljr_rc2 == cs.pc.lja_rc2;
         const size_t smem = list_smem(same, false);
-        auto* k = same ? (energy ? k_forces_lists<true, true> : k_forces_lists<true, false>)
-                       : (energy ? k_forces_lists<false, true> : k_forces_lists<false, false>);
+        const bool all = energy || (excl_all & kTermLJR);  // the form that knows a switched-off repulsion (lj_pair)
+        auto* k = same ? (all ? k_forces_lists<true, true> : k_forces_lists<true, false>)
+                       : (all ? k_forces_lists<false, true> : k_forces_lists<false, false>);
         launch(k, grid, kListThreads, smem, s, dependent, a);
     } else if ((terms & ~(kTermEXV | kTermDH)) == 0) launch_forces_t<kTermEXV | kTermDH>(a, grid, s, per, energy, dependent);
     else if (terms == (kTermLJR | kTermLJA) && cs.lj_same_sigma)

@@ -1676,7 +1676,8 @@ int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 // b+1, b+2 or b+3, the reach of the AICG2+ local contacts, which as gather
 // entries were evaluated by both of their beads; angle b..b+2; dihedral
 // b..b+3, either direction; angles and dihedrals are reversed to increasing
-// order, which leaves the angle and the torsion unchanged).
+// order, which leaves the angle and the torsion unchanged).  A bond of a
+// bead with itself is not (its force is NaN, not another bond's).
 // Chain-local terms come first, sorted by their first bead (stable, so
 // terms on the same beads keep their order), with per-bead start indices;
 // every other term is listed in the gather entries of each of its beads
@@ -1700,7 +1701,7 @@ BondedPlan plan_bonded(const CompiledSystem& c) {
     std::vector<std::pair<int64_t, DihedralTerm>> chd;
     for (BondTerm t : c.bonds) {
         if (t.i > t.j) std::swap(t.i, t.j);
-        if (t.j <= t.i + 3) chb.emplace_back(t.i, t);
+        if (t.i < t.j && t.j <= t.i + 3) chb.emplace_back(t.i, t);
         else ob.push_back(t);
     }
     for (AngleTerm t : c.angles) {

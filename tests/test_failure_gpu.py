@@ -59,3 +59,25 @@ def test_periodic_blow_up_is_reported(gpu):
     with pytest.raises(gpu.OCMError) as ei:
         ctx.step(5)
     assert ei.value.code == 7
+
+
+@pytest.mark.parametrize("bead", [7, 118])
+def test_bond_of_a_bead_with_itself_is_reported(gpu, bead):
+    """Its force is not a number: the batched kernel reports it as the plain
+    path does, wherever the bead lies."""
+    from opencafemol_gb300 import synth
+    spec = synth.go_protein(119, 36)
+    spec.bonds = np.concatenate([spec.bonds, [[bead, bead]]])
+    spec.bond_v0 = np.append(spec.bond_v0, 0.38)
+    spec.bond_k = np.append(spec.bond_k, 1000.0)
+    system = synth.build_system(spec)
+    ctx = gpu.Context(system, gpu.LangevinIntegrator(300.0, 0.1, 0.01, 3))
+    ctx.setPositions(spec.pos)
+    b = gpu.Batch(max_systems=1, max_total_beads=128, max_beads_per_system=128)
+    slot = b.admit(system, spec.pos, seed=1, n_steps=2)
+    for call in (ctx.getState, lambda: b.state(slot)):
+        with pytest.raises(gpu.OCMError) as ei:
+            call()
+        assert ei.value.code == 7
+    b.run(2)
+    assert b.status(slot) == 7

@@ -1504,6 +1504,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_batch(BatchArgs a) {
     // system's results do not depend on the threads that run it (the pair
     // split depends on its bead count alone), so they do not depend on the
     // split either.
+    __syncthreads();  // every thread has read the CTA's claim, whose word is the first half's from here on
     const int half = tid / (THREADS / 2);
     const size_t half_bytes = (a.smem_bytes / 2) & ~(size_t)255;
     const int next_q = split_phase<THREADS / 2, MODE, ENERGY, INTEGRATE>(

@@ -2468,7 +2468,8 @@ void BatchEngine::slot_stats(int64_t slot, int32_t* builds, int32_t* capacity) {
     int b = 0;
     OCM_CK(cudaMemcpy(&b, &sys_.p[slot].builds, sizeof(int), cudaMemcpyDeviceToHost));
     *builds = b;
-    *capacity = sys_host_[slot].maxn;
+    const BatchSys& R = sys_host_[slot];
+    *capacity = R.maxn * pair_split(R.n, split_units(R.cls));  // of the main list, all units of a bead
 }
 
 // Scatter / gather of many slots' states through one pinned staging buffer

@@ -160,3 +160,19 @@ def test_general_terms(gpu, terms, n):
     other = b.admit(system, straight, seed=1, n_steps=1)
     b.set_positions_many([other], spec.pos)
     assert np.array_equal(b.state(other)[0], f)
+
+
+@pytest.mark.parametrize("kind", ["go", "hps", "general"])
+@pytest.mark.parametrize("n", [64, 200, 400])
+def test_list_capacity_is_per_bead(gpu, kind, n):
+    """slot_stats counts the entries of a bead, however many units share
+    them: room for every partner that the positions at admission have."""
+    from opencafemol_gb300 import synth
+    spec = _chain(kind, n, 20 + n)
+    b = gpu.Batch(max_systems=1, max_total_beads=1024, max_beads_per_system=512)
+    slot = b.admit(synth.build_system(spec), spec.pos, seed=1, n_steps=1)
+    reach = 3.5 if kind == "general" else 2.0  # the main list's cutoff
+    d = np.linalg.norm(spec.pos[:, None] - spec.pos[None], axis=2)
+    partners = int((d < reach).sum(axis=1).max()) - 1
+    capacity = b.slot_stats(slot)["list_capacity"]
+    assert partners <= capacity <= n + 32

@@ -141,7 +141,7 @@ class PlainContext {
     void rebuild_charged_rows(cudaStream_t s);
     NeighbourLists neighbour_lists() const;
     size_t list_smem(bool same_sigma, bool build) const;
-    int column_reach(float cut, int reach[2]) const;
+    void column_reach(float cut, int reach[2]) const;
     void alloc_pair_lists();
     bool pair_list_terms() const;
     void leave_pair_lists();

@@ -719,7 +719,6 @@ __global__ void k_chg_list_pairs(int m, const int32_t* __restrict__ idx, const i
 // 22 per launch.  The tiles take 44.
 // ---------------------------------------------------------------------------
 constexpr int kMaxNeighbours = 128;  // so that an entry fits 16 bits
-constexpr int kMaxColumns = 512;     // columns a neighbourhood may span
 constexpr int kListUnits = 8;
 constexpr int kListThreads = 32 * kListUnits;
 constexpr int kMaxUnitEntries = 32 * kMaxNeighbours / kListUnits;  // every staged bead
@@ -2003,7 +2002,6 @@ void PlainContext::rebuild(cudaStream_t s) {
     const int wblocks = div_up(nc * 32, 128);
     const float cut = (float)(tile_cutoff_ + skin) * 1.0001f + 1e-4f;
     const float cut2 = cut * cut;
-    if (int reach[2]; pair_lists_ && column_reach(cut, reach) > kMaxColumns) leave_pair_lists();
     if (pair_lists_) {
         rebuild_pair_lists(s, cut);
         rebuild_charged_rows(s);
@@ -2076,14 +2074,9 @@ void PlainContext::rebuild_pair_lists(cudaStream_t s, float cut) {
 }
 
 // Columns to either side that can hold a neighbour (their gap stays below
-// the cutoff); returns how many columns a neighbourhood spans.
-int PlainContext::column_reach(float cut, int reach[2]) const {
-    int span = 1;
-    for (int a = 0; a < 2; ++a) {
-        reach[a] = (int)((cut + 1e-3) / (cs.box[a] / cell_dims_[a])) + 1;
-        span *= std::min(cell_dims_[a], 2 * reach[a] + 1);
-    }
-    return span;
+// the cutoff).
+void PlainContext::column_reach(float cut, int reach[2]) const {
+    for (int a = 0; a < 2; ++a) reach[a] = (int)((cut + 1e-3) / (cs.box[a] / cell_dims_[a])) + 1;
 }
 
 NeighbourLists PlainContext::neighbour_lists() const {
@@ -2563,7 +2556,9 @@ bool PlainContext::pair_list_terms() const {
 }
 
 // Back to the tiles, for a system whose neighbourhoods do not fit a block
-// (more than kMaxNeighbours clusters or kMaxColumns columns).
+// (more than kMaxNeighbours clusters), until the list options change: new
+// positions do not bring the lists back, so a dense system that is handed
+// frame after frame does not build them in vain for each.
 void PlainContext::leave_pair_lists() {
     pair_lists_ = false;
     clear_graphs();

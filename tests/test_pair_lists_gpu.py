@@ -94,3 +94,38 @@ def test_globule_with_nearly_every_bead_in_range(gpu):
     assert st["masked_tiles"] == 0 and st["tiles"] > 0  # the lists, not the tiles
     ctx.step(20)
     assert np.all(np.isfinite(ctx.getPositions()))
+
+
+def test_neighbourhood_of_many_columns(gpu):
+    """A rod of 17,000 beads along z in a box of 23 x 23 columns, all within
+    the 19 nm cutoff of each other: few of them hold a cluster."""
+    from opencafemol_gb300 import synth
+    from oracle import oracle
+    chains, length = 170, 100
+    n, a = chains * length, 0.47
+    spec = synth.hps_slab(30, 100, (15.0, 15.0, 60.0), slab_width=20.0, seed=6, hps_cutoff=19.0)
+    k = np.arange(n)
+    layer, site = k // 16, k % 16
+    site = np.where(layer % 2, 15 - site, site)
+    y = site // 4
+    x = np.where(y % 2, 3 - site % 4, site % 4)
+    spec.n, spec.box = n, (44.0, 44.0, 520.0)
+    pos = np.stack([21.3 + a * x, 21.3 + a * y, 3.0 + a * layer], 1)
+    spec.pos = (pos + np.random.default_rng(8).normal(scale=0.01, size=pos.shape)).astype(np.float32).astype(np.float64)
+    tile = lambda v: np.resize(v, n)
+    spec.masses = tile(spec.masses)
+    for t in (spec.ljr, spec.lja):
+        t.p0, t.p1 = tile(t.p0), tile(t.p1)
+    spec.dh = None
+    b0 = (np.arange(chains)[:, None] * length + np.arange(length - 1)[None]).ravel()
+    spec.bonds = np.stack([b0, b0 + 1], 1)
+    spec.bond_v0 = np.linalg.norm(spec.pos[b0 + 1] - spec.pos[b0], axis=1)
+    spec.bond_k = np.full(len(b0), spec.bond_k[0])
+    ctx = gpu.Context(synth.build_system(spec), gpu.LangevinIntegrator(spec.temperature, 5.0, 0.001, 7))
+    ctx.setPositions(spec.pos)
+    f, _ = ctx.getState(energy=False)
+    f_ref, _ = oracle.evaluate(spec, cells=0)
+    assert rel_force_err(f, f_ref) <= FORCE_TOL
+    assert ctx.stats()["masked_tiles"] == 0  # the lists
+    ctx.step(10)
+    assert np.all(np.isfinite(ctx.getPositions()))

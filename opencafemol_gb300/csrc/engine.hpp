@@ -150,6 +150,7 @@ class PlainContext {
     void setup_columns(double width);
     BoxD box_d() const;
     float wrap_pad() const;
+    void alloc_tiles();
     void alloc_tile_arrays();
     bool eval(uint32_t groups, bool energy, double* forces, double* slot_energy);
     uint32_t slots_for_groups(uint32_t groups) const;

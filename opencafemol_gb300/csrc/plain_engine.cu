@@ -1778,9 +1778,7 @@ PlainContext::PlainContext(const SystemDesc& d, double temperature, double frict
     bb_c_.alloc(nc); bb_h_.alloc(nc); anc_.alloc(nc); ext_.alloc(nc);
     tile_count_.alloc(nc); tile_start_.alloc(nc + 1); raw_start_.alloc(nc + 1);
     tile_cap_ = std::min<int64_t>(nc * (nc + 1) / 2, std::max<int64_t>(4096, nc * 48));
-    alloc_tile_arrays();
     mask_cap_ = std::max<int64_t>(256, std::min<int64_t>(tile_cap_, nc * 8));
-    masks_.alloc(mask_cap_ * 128);
     mask_count_.alloc(1);
 
     if (reorder) {
@@ -1835,6 +1833,8 @@ PlainContext::PlainContext(const SystemDesc& d, double temperature, double frict
         list_cap_ = 24;
         ljs_.alloc(np);
         alloc_pair_lists();
+    } else {
+        alloc_tiles();
     }
     bonds_.upload(cs.bonds, s);
     angles_.upload(cs.angles, s);
@@ -2232,6 +2232,7 @@ void PlainContext::launch_integrate(cudaStream_t s, int r) {
 void PlainContext::ensure_capacity() {
     // Build once eagerly, read the sizes back and grow the buffers if needed.
     for (int attempt = 0; attempt < 8; ++attempt) {
+        if (!pair_lists_ && masks_.n == 0) alloc_tiles();  // the first tiles of a context that began on lists
         OCM_CK(cudaMemsetAsync(flags_.p, 0, sizeof(int32_t), stream_));
         rebuild(stream_);
         // sizes into pinned words (a pageable copy waits by itself): total,
@@ -2572,6 +2573,13 @@ void PlainContext::set_list_options(int32_t interval, double sk) {
     // the lists hold no Debye-Hueckel: without the charged rows the tiles do
     pair_lists_ = list_.n > 0 && pair_list_terms();
     clear_graphs();
+}
+
+// The tiles' buffers (about 6 KB per cluster), which a context on pair lists
+// does without.
+void PlainContext::alloc_tiles() {
+    alloc_tile_arrays();
+    masks_.alloc(mask_cap_ * 128);
 }
 
 // Every per-tile array, at tile_cap_ entries (candidate and final lists).

@@ -175,7 +175,7 @@ BYTES_INTEGRATE_PER_BEAD = 100
 # dram__bytes_read.sum + dram__bytes_write.sum of one timed k_batch launch of
 # the default workload (100 MD steps of the 512-replica mix), from a
 # `ncu --set full --clock-control none` capture of this script
-K_BATCH_DRAM_BYTES = 21907712 + 512
+K_BATCH_DRAM_BYTES = 21906688 + 1536
 
 
 def measured_hbm_gbs():
@@ -470,7 +470,9 @@ def run_plain_configs(ocm, args):
                      "ns_per_day": steps / t * spec.dt * 86400 * 1e-3, "us_per_step": t / steps * 1e6,
                      "list_builds": int(st["list_builds"]), "tiles": int(st["tiles"]),
                      "charged_pairs": int(st["charged_pairs"]), "tile_cutoff_nm": round(st["tile_cutoff"], 4),
-                     "engine": "one-system batched kernel" if st["one_system"] else "cluster-pair tiles",
+                     "engine": "one-system batched kernel" if st["one_system"] else
+                               "cluster-pair tiles" if st["masked_tiles"] or not st["reordered"] else
+                               "per-bead pair lists",
                      "untimed_relaxation_steps": int(relax)}
     return out
 

@@ -318,7 +318,9 @@ int ocm_context_get_stats(ocm_context* ctx, ocm_context_stats* out);
 int ocm_context_set_list_options(ocm_context* ctx, int32_t rebuild_interval, double skin);
 /* Debug/verification: every pair (i<j, original indices) that the tile list
  * makes the nonbonded kernel test AND that passes the FP32 cutoff test of
- * the largest cutoff the tiles serve (stats.tile_cutoff), followed, when
+ * the largest cutoff the tiles serve (stats.tile_cutoff); with per-bead lists
+ * in the tiles' place, their pairs that pass that test and the pairs they
+ * leave out as excluded, from the exclusions; followed, when
  * Debye-Hueckel runs on its own charged-pair list (stats.charged_split),
  * by the listed charged pairs that pass its FP32 cutoff test; written to
  * out_pairs.  Used to prove the lists are bit-exact against brute force. */
@@ -383,7 +385,9 @@ int ocm_batch_set_balanced(ocm_batch* batch, int on);
  * systems a CTA claims have at most `beads` beads, the CTA splits into two
  * groups of half its threads, each with half of its shared memory,
  * advancing two systems at a time (default 512; 0 = never split; capped so
- * that a system's state fits half of the CTA's shared memory). */
+ * that a system's state fits half of the CTA's shared memory).  With at
+ * least four systems per CTA a group divides once more, by the same rule, at
+ * systems of at most 96 beads. */
 int ocm_batch_set_split(ocm_batch* batch, int32_t beads);
 /* Wait for the last launch; *status = OCM_OK, or OCM_ERR_NONFINITE if the
  * slot's system blew up (it is no longer advanced; its state is the one of

@@ -82,7 +82,8 @@ constexpr int kSortBuilds = 4;
 // 50..800 beads 2.92 -> 2.30 ms, 300 disordered chains 6.74 -> 1.95 ms, 24
 // proteins of 30..200 beads 0.84 -> 0.56 ms; per 50 steps 160 AICG2+
 // proteins of 800..2000 beads 3.94 -> 2.86 ms (these also through bonds kept
-// chain-local to three positions).
+// chain-local to three positions).  With what followed: 2.08, 1.90, 0.57 and
+// 2.71 ms.
 constexpr int kClassGo = 0;
 constexpr int kClassHps = 1;
 constexpr int kClassGeneral = 2;
@@ -111,9 +112,9 @@ __host__ __device__ __forceinline__ int pair_split(int n, int units) {
 }
 // Units a small system is split into.  Every pass costs about 150 instructions
 // beside its entries, so the short excluded-volume entries want fewer units
-// (against 512: 24 small proteins 549 -> 523 us, 1400 peptides 2.26 -> 2.04
+// (against 512: 24 small proteins 547 -> 522 us, 1400 peptides 2.03 -> 1.71
 // ms per 100 steps), the longer Lennard-Jones ones more (256 against 512:
-// 300 disordered chains 1.85 against 1.76 ms).
+// 300 disordered chains 1.82 against 1.75 ms).
 __host__ __device__ __forceinline__ int split_units(int cls) { return cls == 0 ? 256 : kSplitMost; }
 __host__ __device__ __forceinline__ int charged_units(int cls) { return split_units(cls) / 4; }
 

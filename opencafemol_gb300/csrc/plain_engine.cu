@@ -1,16 +1,18 @@
 // plain_engine.cu - the plain single-system path.
 //
-// Per step: one fused force kernel (cluster-pair tiles for the pair terms,
-// segments for bonds / Go / Gaussian / capped-Go contacts, angles,
-// dihedrals and, when Debye-Hueckel reaches further than the other pair
-// terms, its per-bead charged rows, all in one grid) and one Langevin kernel
-// that also zeroes the fixed-point force buffer.  Every `rebuild_interval`
-// steps the cluster layout and the lists are rebuilt:
+// Per step: one fused force kernel (per-bead pair lists over staged neighbour
+// clusters for the Lennard-Jones terms of large periodic systems, otherwise
+// cluster-pair tiles for the pair terms; segments for bonds / Go / Gaussian /
+// capped-Go contacts, angles, dihedrals and, when Debye-Hueckel reaches
+// further than the other pair terms, its per-bead charged rows, all in one
+// grid) and one Langevin kernel that also zeroes the fixed-point force buffer.
+// Every `rebuild_interval` steps the cluster layout and the lists are rebuilt:
 //   cell keys (x-y columns, z slices; periodic systems) -> counting sort
-//   with in-cell ranks -> gather into cluster order with anchored offsets
-//   -> bounding boxes and anchors -> candidate tiles (count / scan / fill)
-//   -> exact pruning -> compaction with per-tile anchor shifts ->
-//   exclusion masks; charged-bead cells -> charged rows.
+//   with in-cell ranks -> clusters (cluster order, bounding boxes, anchored
+//   offsets) -> neighbour clusters and per-bead lists in one kernel, or
+//   candidate tiles (count / scan / fill) -> exact pruning -> compaction with
+//   per-tile anchor shifts -> exclusion masks; charged-bead cells -> charged
+//   rows.
 // A chunk of steps (rebuild + steps) is captured once into a CUDA graph.
 #include <cuda_runtime.h>
 

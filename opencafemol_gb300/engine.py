@@ -23,8 +23,9 @@ class Context:
     """OpenMM's Context + LangevinIntegrator as the reference's Simulator
     drives them.  ``engine`` picks the kernels of ``step``: "auto" (a
     non-periodic system of at most 512 beads as a one-system persistent
-    launch of the batched kernel, anything else on the cluster-pair tiles),
-    "tiles" or "one_system"."""
+    launch of the batched kernel, anything else on cluster-pair tiles or, for
+    the Lennard-Jones terms of large periodic systems, on per-bead lists),
+    "tiles" (the latter for every system) or "one_system"."""
 
     ENGINES = {"auto": 0, "tiles": 1, "one_system": 2}
 

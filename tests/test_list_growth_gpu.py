@@ -146,3 +146,24 @@ def test_overlapping_launches_follow_the_oracle(gpu, kind):
     assert moved > 0.02
     assert np.abs(ctx.getPositions() - x).max() <= 1e-4 * moved
     assert np.abs(ctx.getVelocities() - v).max() <= 1e-4 * np.abs(v).max()
+
+
+def test_tiles_until_the_options_change(gpu):
+    """A context that went to the tiles stays there for new positions, and
+    goes back to the lists with its options: the same forces from both."""
+    from opencafemol_gb300 import synth
+    edge = 56.0
+    spec = synth.hps_slab(46, 97, (15.0, 15.0, 60.0), slab_width=30.0, seed=7, hps_cutoff=4.0)
+    spec.dh, spec.box = None, (edge, edge, edge)
+    ctx = gpu.Context(synth.build_system(spec), gpu.LangevinIntegrator(0.0, 1.0, 0.002, 7))
+    sparse = _cube(spec, 1.2, edge)
+    forces = []
+    for positions, options, lists in ((sparse, False, True), (_cube(spec, 0.55, edge), False, False),
+                                      (sparse, False, False), (sparse, True, True)):
+        if options:
+            ctx.set_list_options(skin=ctx.stats()["skin"])
+        ctx.setPositions(positions)
+        forces.append(ctx.getState(energy=False)[0])
+        assert (ctx.stats()["masked_tiles"] == 0) == lists
+    assert np.array_equal(forces[0], forces[3])
+    assert rel_force_err(forces[2], forces[0]) <= FORCE_TOL
